@@ -75,6 +75,7 @@ struct Control {
     int pad;
     int expert_rows[kMaxLocalExperts];   // copy of the counters of the last call (diagnostics)
     int splitk_ticket[kSplitKSlots];     // per-tile arrival counters of the split-K reduction (self-clearing)
+    int unit_ticket[2];                  // next work unit of the fused expert GEMMs (zeroed by the routing kernel's scan)
     int push_done;                       // combine-and-push CTAs finished (ticket, self-clearing)
     unsigned dec_count;                  // arrival counters of the decode kernel's two grid barriers
     unsigned dec_phase;                  // (cleared by CTA 0 of each launch, see decode.cu)
@@ -129,6 +130,7 @@ struct Workspace {
     int4* tile_info;        // [max_tiles] per 128-row tile: {local expert, first tile of that expert,
                             //             tiles of that expert, routed rows of that expert}
     int* num_tiles;         // [1]
+    unsigned* tile_done;    // [max_tiles] GEMM1 epilogue warps that have finished a tile of this row tile
     int* expert_map;        // [256] global expert -> local index or -1 (table placement only)
     int* topk_idx;          // [T,8] global expert ids in selection order
     float* topk_weight;     // [T,8] normalised weights (before routed_scaling_factor)
@@ -148,6 +150,12 @@ struct Workspace {
     int max_tiles;
     Geometry geo;
     int w_tiled;            // the GEMMs' weight map covers the tile-ordered copy (one 32 KB piece per tile and K block)
+};
+
+// Tensor maps of one pair of GEMM launches (host addresses of CUtensorMap objects): packed activations and
+// weights of GEMM1 and GEMM2, and GEMM2's output rows.
+struct GemmMaps {
+    const void *a1, *w1, *a2, *w2, *y;
 };
 
 }  // namespace moe

@@ -28,9 +28,9 @@ int encode_rows_1k_map(void*, const void*, uint64_t, uint64_t, uint32_t);
 int encode_out_bf16_map(void*, void*, uint64_t, uint64_t);
 size_t tensor_map_bytes();
 cudaError_t configure_gemm_kernels();
-cudaError_t launch_grouped_gemm(int, const void*, const void*, const void*, const Workspace&, const float*, int, int, int, int,
-                                cudaStream_t);
-int gemm_tiles_n(int mode, const Geometry& geo);
+cudaError_t launch_splitk_gemm(int, const GemmMaps&, const Workspace&, const float*, int, int, cudaStream_t);
+cudaError_t configure_expert_gemms();
+cudaError_t launch_expert_gemms(const GemmMaps&, const Workspace&, const float*, const float*, int, int, int, int, cudaStream_t);
 size_t packed_scale_floats(int mode, int num_experts, const Geometry& geo);
 cudaError_t launch_repack_weight_scales(const float*, const float*, float*, float*, int, const Geometry&, cudaStream_t);
 cudaError_t launch_tile_weights(int, const void*, void*, int, const Geometry&, int, cudaStream_t);
@@ -65,7 +65,7 @@ struct Carve {
 };
 
 struct Layout {
-    size_t ctrl, expert_offset, tile_info, num_tiles, expert_map, topk_idx, topk_weight, pair_count, pair_code,
+    size_t ctrl, expert_offset, tile_info, tile_done, num_tiles, expert_map, topk_idx, topk_weight, pair_count, pair_code,
         pair_weight, pair_row, row_token, a1, sfa1, a2, sfa2, y, splitk, sw1_packed, sw2_packed, total;
     int m_cap, max_tiles;
 };
@@ -82,6 +82,7 @@ Layout make_layout(int T, int E, const Geometry& geo = kReferenceGeometry)
     L.ctrl = c.take(sizeof(Control));
     L.expert_offset = c.take(sizeof(int) * (kMaxLocalExperts + 1));
     L.tile_info = c.take(sizeof(int4) * L.max_tiles);
+    L.tile_done = c.take(sizeof(unsigned) * L.max_tiles);
     L.num_tiles = c.take(sizeof(int) * 4);
     L.expert_map = c.take(sizeof(int) * kNumExperts);
     L.topk_idx = c.take(sizeof(int) * (size_t)T * kTopK);
@@ -333,17 +334,27 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
     const int split_k = (T <= 4 && ref_geo) ? 1 : 0;   // 4 = kSplitKMaxRows of the GEMM kernel
     // at most 64 tokens (an expert then has at most 64 rows): 64-row activation boxes and a fourth operand stage
     const int small_a = (h->opt_small_batch_ring && T > 4 && T <= 64 && ref_geo) ? 1 : 0;
-    // one persistent CTA per SM; CTAs without work leave at once, spare ones take split-K units
-    auto ctas = [&](int) { return h->num_sms; };
     if (e == cudaSuccess && stop >= 2) e = launch_permute(a.hidden_states, a.hidden_states_scale, h->ws, T, stream);
     mark(3);
-    if (e == cudaSuccess && stop >= 3)
-        e = launch_grouped_gemm(1, small_a ? h->tmap_a1_small : h->tmap_a1, tiled ? h->tmap_w1_tiled : h->tmap_w1, h->tmap_y,
-                                gemm_ws, h->sw1_packed, h->opt_exact_silu, ctas(1), split_k, small_a, stream);
-    mark(4);
-    if (e == cudaSuccess && stop >= 4)
-        e = launch_grouped_gemm(2, small_a ? h->tmap_a2_small : h->tmap_a2, tiled ? h->tmap_w2_tiled : h->tmap_w2, h->tmap_y,
-                                gemm_ws, h->sw2_packed, 0, ctas(2), split_k, small_a, stream);
+    const GemmMaps maps = {small_a ? h->tmap_a1_small : h->tmap_a1, tiled ? h->tmap_w1_tiled : h->tmap_w1,
+                           small_a ? h->tmap_a2_small : h->tmap_a2, tiled ? h->tmap_w2_tiled : h->tmap_w2, h->tmap_y};
+    // one persistent CTA per SM; CTAs without work leave at once
+    auto gemms = [&](int phases) {
+        return launch_expert_gemms(maps, gemm_ws, h->sw1_packed, h->sw2_packed, h->opt_exact_silu, phases, h->num_sms, small_a, stream);
+    };
+    if (split_k) {
+        if (e == cudaSuccess && stop >= 3)
+            e = launch_splitk_gemm(1, maps, gemm_ws, h->sw1_packed, h->opt_exact_silu, h->num_sms, stream);
+        mark(4);
+        if (e == cudaSuccess && stop >= 4) e = launch_splitk_gemm(2, maps, gemm_ws, h->sw2_packed, 0, h->num_sms, stream);
+    } else if (ev || stop == 3) {
+        // the same kernel cut between the two GEMMs, for callers that time or read what lies between them
+        if (e == cudaSuccess && stop >= 3) e = gemms(1);
+        mark(4);
+        if (e == cudaSuccess && stop >= 4) e = gemms(2);
+    } else {
+        if (e == cudaSuccess && stop >= 4) e = gemms(3);
+    }
     mark(5);
     if (e == cudaSuccess && stop >= 5 && finalize) {
         if (ex) {
@@ -505,6 +516,7 @@ int moe_fp8_b200_create_shaped(moe_fp8_b200_handle* out, int device, int max_tok
     w.ctrl = reinterpret_cast<Control*>(h->base + L.ctrl);
     w.expert_offset = reinterpret_cast<int*>(h->base + L.expert_offset);
     w.tile_info = reinterpret_cast<int4*>(h->base + L.tile_info);
+    w.tile_done = reinterpret_cast<unsigned*>(h->base + L.tile_done);
     w.num_tiles = reinterpret_cast<int*>(h->base + L.num_tiles);
     w.topk_idx = reinterpret_cast<int*>(h->base + L.topk_idx);
     w.topk_weight = reinterpret_cast<float*>(h->base + L.topk_weight);
@@ -529,6 +541,7 @@ int moe_fp8_b200_create_shaped(moe_fp8_b200_handle* out, int device, int max_tok
     e = cudaMemset(h->base, 0, L.topk_idx);
     if (e == cudaSuccess) e = cudaMemset(w.row_token, 0xff, sizeof(int) * (size_t)L.m_cap);
     if (e == cudaSuccess) e = configure_gemm_kernels();
+    if (e == cudaSuccess) e = configure_expert_gemms();
     int mr = 0;
     if (e == cudaSuccess) {
         if (tensor_map_bytes() > sizeof(h->tmap_a1)) mr = -100;
@@ -1016,7 +1029,7 @@ int moe_fp8_b200_check(moe_fp8_b200_handle h, void* stream)
     }
     if (st[0] != kStatusOk)
         return fail(h, MOE_FP8_B200_ERR_DEVICE, "device status %d (detail %d): %s", st[0], st[1],
-                    st[0] == kStatusGemm1Timeout   ? "GEMM1 gave up on a bounded wait"
+                    st[0] == kStatusGemm1Timeout   ? "the expert GEMMs (or GEMM1) gave up on a bounded wait"
                     : st[0] == kStatusGemm2Timeout ? "GEMM2 gave up on a bounded wait"
                     : st[0] == kStatusRowOverflow  ? "routed rows exceed the workspace capacity"
                     : st[0] == kStatusExchangeTimeout ? "a peer rank's rows did not arrive within the wait limit"

@@ -54,13 +54,17 @@ __device__ __forceinline__ void scan_tiles_block(const Workspace& ws, int num_lo
         ws.expert_offset[num_local_experts] = total * kTileM;
         ws.num_tiles[0] = total;
         ws.ctrl->blocks_done = 0;
+        ws.ctrl->unit_ticket[0] = ws.ctrl->unit_ticket[1] = 0;
         // the status word is sticky: the first failure stays until the host has read it
         if (overflow && atomicCAS(&ws.ctrl->status, kStatusOk, kStatusRowOverflow) == kStatusOk)
             ws.ctrl->status_detail = warp_base + incl;
     }
     if (!overflow && e < num_local_experts) {
         const int4 info = make_int4(e, base, k, m);
-        for (int j = 0; j < k; ++j) ws.tile_info[base + j] = info;
+        for (int j = 0; j < k; ++j) {
+            ws.tile_info[base + j] = info;
+            ws.tile_done[base + j] = 0;
+        }
     }
 }
 
