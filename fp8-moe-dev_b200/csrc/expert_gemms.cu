@@ -178,12 +178,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
         prefetch_tmap(&tmap_w2);
         prefetch_tmap(&tmap_y);
     }
-    // Everything above is independent of earlier kernels; from here on their results are read.
-    pdl_wait();
-    const int row_tiles = ws.num_tiles[0];
-    const int units1 = row_tiles * tiles_n1, units_all = units1 + row_tiles * tiles_n2;
-    const int unit_begin = phases == 2 ? units1 : 0, unit_end = phases == 1 ? units1 : units_all;
-    if ((int)blockIdx.x >= unit_end - unit_begin) return;  // nothing for this CTA: leave before touching TMEM
     if (warp == 2) {
         tmem_alloc(smem_u32(&sh->tmem_base), kTmemCols);
         tmem_relinquish();
@@ -200,7 +194,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
         setmaxnreg_dec<56>();
         if (warp == 0 && lane == 0) {
             // ------------------------------------------------------------ producer
+            // The kernel in front of this one in the chain (permute, or the GEMM1 half) triggers the launch only
+            // once the routing kernel's results are complete, so units can be drawn and looked up and the first
+            // weights requested while it still runs; its own results are read after pdl_wait().
             int* ticket = &ws.ctrl->unit_ticket[phases == 2 ? 1 : 0];
+            const int row_tiles = __ldcg(ws.num_tiles);
+            const int first_ticket = atomicAdd(ticket, 1);
+            const int units1 = row_tiles * tiles_n1, units_all = units1 + row_tiles * tiles_n2;
+            const int unit_begin = phases == 2 ? units1 : 0, unit_end = phases == 1 ? units1 : units_all;
             const unsigned done_count = 2u * (unsigned)tiles_n1;   // both epilogue warps of every GEMM1 unit of the row tile
             uint32_t it = 0, ui = 0;
             bool ok = true;
@@ -219,11 +220,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
                 ++ui;
                 return true;
             };
-            int id = unit_begin + atomicAdd(ticket, 1);
+            int id = unit_begin + first_ticket;
             UnitDesc d;
             d.mode = 0;
             if (id < unit_end) d = desc_of(record_of(id), id);
             bool rows_ready = phases == 2;   // an earlier launch finished all GEMM1 units
+            bool first = true;
             while (ok && id < unit_end) {
                 const bool g1 = d.mode == 1;
                 const CUtensorMap* map_a = g1 ? &tmap_a1 : &tmap_a2;
@@ -247,10 +249,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
                     }
                 };
                 int pre = 0;   // K blocks whose weights have been requested ahead of the rows
+                const int lim = kblocks < kStages ? kblocks : kStages;
+                if (first) {
+                    while (pre < lim) load_weights(pre++);
+                    pdl_wait();
+                    first = false;
+                }
                 if (!g1) {
                     if (!rows_ready) {
                         const unsigned* done = ws.tile_done + d.row0 / kTileM;
-                        const int lim = kblocks < kStages ? kblocks : kStages;
                         const uint64_t t0 = global_timer_ns();
                         while (ld_acquire_gpu_u32(done) < done_count) {
                             if (pre < lim) {
@@ -439,6 +446,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
     } else {
         // ---------------------------------------------------------------- promotion
         setmaxnreg_inc<224>();
+        pdl_wait();   // the packed rows' scales
         const int ew = warp - 4;
         const int h = ew >> 2;       // which 128 of the tile's 256 accumulator columns
         const int q = warp & 3;      // TMEM lane quarter this warp may read

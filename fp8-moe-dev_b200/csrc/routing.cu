@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_kernel(
 {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kPermuteWarps + (threadIdx.x >> 5);
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();   // after the wait: the expert GEMMs rely on the routing kernel being complete when they start
     if (t >= T) return;
     const int n_pairs = (ws.num_tiles[0] == 0) ? 0 : ws.pair_count[t];
     if (lane < kTopK) {   // the token's packed rows, for the fused exchange
@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_generic_kerne
 {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kPermuteWarps + (threadIdx.x >> 5);
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();   // after the wait: the expert GEMMs rely on the routing kernel being complete when they start
     if (t >= T) return;
     const int n_pairs = (ws.num_tiles[0] == 0) ? 0 : ws.pair_count[t];
     if (lane < kTopK) {
