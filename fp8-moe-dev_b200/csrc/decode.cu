@@ -1,30 +1,32 @@
-// Decode path: the whole layer for a batch of at most eight tokens as ONE cooperative kernel.
+// Decode path: the layer for a batch of at most eight tokens as one persistent kernel plus the combine.
 //
 // With a handful of tokens every active expert has at most eight rows, the layer is nothing
 // but streaming the active experts' weights once (44 MB per expert), and what the staged
-// chain of five kernels spends between those streams -- four kernel boundaries, the permute,
-// the padding of every expert to a 128-row tensor-core tile, TMEM set-up, the cross-CTA
-// split-K hand-over -- costs more than the streams themselves.  Here:
-//   * every CTA routes the (<= 8) tokens itself, with the same warp-per-token routine as the
-//     staged chain, and derives the same active-expert table, so nothing has to be exchanged
-//     before the first weight byte is requested;
+// chain of kernels spends between those streams -- kernel boundaries, the permute, the padding of every
+// expert to a 128-row tensor-core tile, TMEM set-up -- costs more than the streams themselves.  Here:
+//   * every CTA routes the (<= 8) tokens itself, with the same selection as the staged chain, and derives
+//     the same active-expert table, so nothing has to be exchanged before the first weight byte is
+//     requested;
 //   * phase 1 (GEMM1 + SwiGLU): a unit is 8 SwiGLU columns of one active expert = 8 linear +
 //     8 gated rows of W1, i.e. exactly one 16-row A tile of the warp-level
 //     mma.sync.m16n8k32 (e4m3 x e4m3 -> fp32), with the expert's <= 8 token rows as the 8-wide
 //     B tile.  The weights arrive by TMA, 16 rows x 1 KB per step (two boxes of 8 rows in
-//     phase 1, one of 16 in phase 2) through a ring of four steps per half CTA; the warps
-//     split K, promote per 128-K block with the two scales like the staged kernel, and meet
-//     in shared memory.  (Per-thread loads and per-row bulk copies both left the HBM two
-//     thirds idle: the first for the loads in flight a thread can hold, the second for the
-//     rate at which one thread can issue sixteen copies per step.)
+//     phase 1, one of 16 in phase 2) through a ring of four or five steps per half CTA, fed by a
+//     producer warp per half; eight warps split a step along K, promote per 128-K block with the two scales
+//     like the staged kernel, and meet in shared memory.  (Per-thread loads and per-row bulk copies both
+//     left the HBM two thirds idle: the first for the loads in flight a thread can hold, the second for the
+//     rate at which one thread can issue sixteen copies per step.  A consumer thread as producer left it
+//     at 5.3 TB/s: freed slots waited for that thread's own share of the step and of the unit's sum.)
 //     In the accumulator layout a thread owns the linear and the gated value of the same
 //     (column, token), so SwiGLU needs no exchange.  v = silu(gate) * lin goes to a small
 //     fp32 scratch (the 1x128 requantisation needs whole 128-column blocks, which span units);
-//   * grid barrier; phase 2 (GEMM2): each CTA requantises the rows of its expert from the
-//     scratch (same arithmetic as the staged epilogue), streams 16 rows of W2 per unit the
-//     same way, and writes bf16 y rows; grid barrier; phase 3 is the weighted combine.
-// The first weights of phase 2 are requested before the barrier, so the barrier and the
-// requantisation hide behind their latency.  Every wait (mbarriers, grid barriers) is bounded.
+//   * phase 2 (GEMM2): a worker waits for its expert's rows in the scratch, requantises them (same arithmetic as
+//     the staged epilogue), streams 16 rows of W2 per unit the same way, and writes bf16 y rows; the first weights are requested before that wait, so the wait
+//     and the requantisation hide behind their latency;
+//   * the weighted combine is a kernel of its own (decode_combine_kernel): it is resident before this one ends,
+//     so its start costs no more than a grid barrier would, and meanwhile the CTAs of the next
+//     layer's decode kernel, which need this one's shared memory, can move in.
+// Every wait is bounded.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -40,8 +42,9 @@ namespace moe {
 
 namespace {
 
-constexpr int kDecWarps = 16;
-constexpr int kDecThreads = kDecWarps * 32;
+constexpr int kDecWarps = 16;                           // consumer warps; two producer warps follow
+constexpr int kConsumers = kDecWarps * 32;
+constexpr int kDecThreads = kConsumers + 64;
 constexpr int kHalfWarps = 8;                           // the CTA works as two halves of 8 warps
 constexpr int kHalfThreads = kHalfWarps * 32;
 constexpr int kDecMaxActive = kDecodeMaxTokens * kTopK; // 64 (token, expert) pairs at most
@@ -58,21 +61,33 @@ constexpr int kStepStride = kStepK;                     // rows of a step lie de
 constexpr int kStepBytes = kStepRows * kStepK;          // 16 KB arrive per step
 constexpr int kG1Steps = kHidden / kStepK;              // 7 per phase-1 unit
 constexpr int kG2Steps = kInter / kStepK;               // 2 per phase-2 unit
-constexpr int kRing = 4;                                // steps in flight per half
-constexpr int kCoopRouteTokens = 2;                     // up to here the CTA routes a token together
+constexpr int kRing = 4;                                // steps in flight per half ...
+constexpr int kRingFew = 5;                             // ... and with at most kFewTokens tokens, whose rows leave room
+constexpr int kFewTokens = 4;
+constexpr int kCoopRouteTokens = 3;                     // up to here the CTA's warps route the tokens together
 static_assert(kHidden % kStepK == 0 && kInter % kStepK == 0, "K splits into whole steps");
-static_assert(2 * kDecodeMaxTokens * kA2Stride <= kDecodeMaxTokens * kHidStride, "phase 2 rows reuse the hidden-row area");
+
+// Shared-memory pool: the hidden rows of all tokens (phase 2: each half's requantised rows of its expert), then
+// the two weight rings.
+__host__ __device__ constexpr int rows_tokens(int T) { return T <= kFewTokens ? kFewTokens : kDecodeMaxTokens; }
+constexpr int kPoolFew = kFewTokens * kHidStride + 2 * kRingFew * kStepBytes;
+constexpr int kPoolAll = kDecodeMaxTokens * kHidStride + 2 * kRing * kStepBytes;
+constexpr int kPoolBytes = kPoolFew > kPoolAll ? kPoolFew : kPoolAll;
+static_assert(kDecodeMaxTokens * kHidStride % 128 == 0 && kFewTokens * kHidStride % 128 == 0, "ring slots are 128-byte aligned");
+// half 1's rows lie rows_tokens(T) rows behind half 0's; the MMAs read eight rows from either start
+static_assert((kFewTokens + 8) * kA2Stride <= kFewTokens * kHidStride && 16 * kA2Stride <= kDecodeMaxTokens * kHidStride,
+              "phase 2 rows reuse the hidden-row area");
+static_assert(2 * kDecodeMaxTokens * kNumExperts * 4 <= 2 * kRing * kStepBytes, "routing scratch fits the idle rings");
 
 struct DecodeShared {
-    int n_active, n_rows, abort, pad;
+    int n_rows, abort;
     int pair_count[kDecodeMaxTokens];
-    int pair_le[kDecodeMaxTokens][kTopK];
-    int pair_slot[kDecodeMaxTokens][kTopK];
-    int pair_row[kDecodeMaxTokens][kTopK];
-    float pair_w[kDecodeMaxTokens][kTopK];
+    int pair_le[kDecMaxActive];                            // [token][pair] local expert, -1 past the token's pairs
+    int pair_first[kDecMaxActive];                         // entry of that expert's first use
+    float pair_w[kDecMaxActive];
     int act_expert[kDecMaxActive], act_m[kDecMaxActive], act_row0[kDecMaxActive];
     int act_tok[kDecMaxActive][kDecodeMaxTokens];
-    int expert_slot[kMaxLocalExperts];
+    int expert_m[kMaxLocalExperts];
     // routing scratch
     float r_gscore[kDecodeMaxTokens][kNumGroups];
     int r_kept[kDecodeMaxTokens][kTopKGroup];
@@ -81,22 +96,32 @@ struct DecodeShared {
     float r_sel[kDecodeMaxTokens][kTopK];
     float hid_scale[kDecodeMaxTokens][kHiddenBlocks];      // [token][kb]
     float a2_scale[2][kDecodeMaxTokens][kInterBlocks];     // per half: [slot][kb] of the requantised rows
-    alignas(8) uint64_t full_bar[2][kRing];
-    alignas(8) uint64_t empty_bar[2][kRing];
+    alignas(16) int4 step_desc[2][kRingFew];               // {unit, step, next unit or -1, -}; unit -1: no more
+    alignas(8) uint64_t full_bar[2][kRingFew];
+    alignas(8) uint64_t empty_bar[2][kRingFew];
     alignas(8) uint64_t hid_bar;
     alignas(16) float red[2][2][kHalfWarps][128];          // per half, by unit parity: the warps' partial sums
-    // phase 1: the hidden rows of all tokens; phase 2: each half's requantised rows of its expert
-    alignas(128) uint8_t rows[kDecodeMaxTokens * kHidStride];
-    alignas(128) uint8_t wring[2][kRing][kStepRows * kStepStride];
+    alignas(128) uint8_t pool[kPoolBytes];
 };
 static_assert(sizeof(DecodeShared) <= 227 * 1024, "decode kernel shared memory");
 
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const unsigned* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// The SwiGLU scratch is its own flag: between launches every word holds kAbsent, a NaN that no arithmetic here
+// produces (the hardware's NaN results are 0x7fffffff); phase 2 re-reads a word until it holds something else.
+// A flag per expert would need a fence behind every unit's stores (measured: 20 % of the kernel).
+constexpr uint32_t kAbsent = 0xffffffffu;
+__device__ __forceinline__ float4 ld_relaxed_gpu(const float* p) {
+    float4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
     return v;
+}
+__device__ __forceinline__ void st_relaxed_gpu(float* p, float v) {
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ bool is_there(const float4& v) {
+    return __float_as_uint(v.x) != kAbsent && __float_as_uint(v.y) != kAbsent && __float_as_uint(v.z) != kAbsent &&
+           __float_as_uint(v.w) != kAbsent;
 }
 
 // Untiled bulk copy global -> shared memory of this CTA, completion counted on an mbarrier.
@@ -135,31 +160,35 @@ __device__ __forceinline__ void mma_block(float (&acc)[4], const uint8_t* arow, 
     }
 }
 
-// All CTAs of the (cooperative, co-resident) grid meet here: one release-add on `counter`, then
-// acquire-polls until all have arrived.  The kernel has two barriers on two counters; CTA 0 clears
-// the second one before it arrives at the first (nobody can reach the second barrier earlier) and
-// the first one after it has passed the second (everybody has left the first by then), so a launch
-// finds and leaves the state it needs without a generation word.  Bounded: a CTA that waits longer
-// than the limit records the failure and returns false; its peers run into the same limit.
-__device__ __forceinline__ bool grid_barrier(unsigned* counter, Control* ctrl, DecodeShared* sh)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-        const uint64_t t0 = global_timer_ns();
-        uint32_t it = 0;
-        while (ld_acquire_gpu(counter) < gridDim.x) {
-            if ((++it & 0x3fu) == 0u && global_timer_ns() - t0 > kWaitLimitNs) {
-                atomicCAS(&ctrl->status, kStatusOk, kStatusDecodeTimeout);
-                sh->abort = 1;
-                break;
-            }
+// How the work is drawn.  Workers (half CTAs) draw tickets from a counter; a ticket stands for a run of
+// consecutive units.  Of each phase the first tickets, one per worker, stand for long runs (three quarters of
+// the phase: few changes of expert, whose rows phase 2 has to requantise again), the rest for short ones that
+// even out how fast the workers get their weights.  All of phase 1 is drawn before phase 2, and phase 2 waits
+// only for phase-1 units, i.e. for workers that are running: the waits end whatever part of the grid is
+// resident, so the launch needs no co-residency guarantee (a cooperative launch starts 3 us later here: it does
+// not overlap its predecessor's end).
+struct PhasePlan {
+    int units, in_runs, runs, rest_run, tickets;
+    __device__ __forceinline__ void make(int n, int workers) {
+        units = n;
+        in_runs = n >= 2 * workers ? n / 4 * 3 : 0;
+        runs = in_runs > 0 ? workers : 0;
+        const int rest = n - in_runs;
+        rest_run = rest / (workers * 6);
+        if (rest_run < 1) rest_run = 1;
+        tickets = runs + (rest + rest_run - 1) / rest_run;
+    }
+    __device__ __forceinline__ void range(int ticket, int& begin, int& end) const {
+        if (ticket < runs) {
+            begin = (int)((long long)in_runs * ticket / runs);
+            end = (int)((long long)in_runs * (ticket + 1) / runs);
+        } else {
+            begin = in_runs + (ticket - runs) * rest_run;
+            end = begin + rest_run < units ? begin + rest_run : units;
         }
     }
-    __syncthreads();
-    return sh->abort == 0;
-}
+};
+constexpr int kPhase2Bit = 1 << 20;   // unit numbers of phase 2 carry it
 
 __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
     DecodeArgs a, const __grid_constant__ CUtensorMap tmap_w1, const __grid_constant__ CUtensorMap tmap_w2, Workspace ws)
@@ -171,33 +200,46 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
     const int T = a.T, E = a.num_local_experts;
     const bool clocked = blockIdx.x == 0 && tid == 0;
     auto stamp = [&](int i) { if (clocked) ws.ctrl->dec_time[i] = global_timer_ns(); };
+    volatile int* abort_flag = &sh->abort;
+
+    // Set-up that depends on no earlier kernel, while the predecessor in the stream drains: barriers, and
+    // requests that bring the call's small inputs from HBM into L2 (the weights of the layers before have
+    // pushed them out; a prefetch returns no value, so it may run ahead of the kernel that writes them).
+    pdl_launch_dependents();
+    if (tid == 0) {
+        sh->abort = 0;
+        prefetch_tmap(&tmap_w1);
+        prefetch_tmap(&tmap_w2);
+        mbar_init(smem_u32(&sh->hid_bar), 1);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < kRingFew; ++j) {
+                mbar_init(smem_u32(&sh->full_bar[h][j]), 1);
+                mbar_init(smem_u32(&sh->empty_bar[h][j]), kHalfWarps);
+            }
+        fence_mbar_init();
+    }
+    if (tid < T * 8) prefetch_l2(a.logits + (size_t)tid * 32);
+    else if (tid >= 64 && tid < 68) prefetch_l2(a.bias + (size_t)(tid - 64) * 64);
+    else if (tid >= 128 && tid < 128 + kHiddenBlocks) prefetch_l2(a.hscale + (size_t)(tid - 128) * T);
+    else if (tid >= 192 && tid < 192 + kHidden / 128) {
+        for (int t = 0; t < T; ++t) prefetch_l2(a.hidden + (size_t)t * kHidden + (size_t)(tid - 192) * 128);
+    }
+    pdl_wait();
     // A failure that an earlier launch recorded stays in the status word until the host has read it
     // (moe_fp8_b200_check clears it together with any arrival counts that launch left on the grid
     // barriers).  Until then this kernel does nothing: with stale counts its barriers would open early.
     // Every CTA reads the same word; within one launch it can only change after a full wait limit.
     if (__ldcg(&ws.ctrl->status) != kStatusOk) return;
     stamp(0);
-    volatile int* abort_flag = &sh->abort;
 
     // The tokens' hidden rows start moving before anything else: nothing depends on routing here.
     if (tid == 0) {
-        sh->abort = 0;
-        prefetch_tmap(&tmap_w1);
-        prefetch_tmap(&tmap_w2);
         const uint32_t hb = smem_u32(&sh->hid_bar);
-        mbar_init(hb, 1);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int j = 0; j < kRing; ++j) {
-                mbar_init(smem_u32(&sh->full_bar[h][j]), 1);
-                mbar_init(smem_u32(&sh->empty_bar[h][j]), kHalfWarps);
-            }
-        fence_mbar_init();
         mbar_expect_tx(hb, (uint32_t)T * kHidden);
         for (int t = 0; t < T; ++t)
-            bulk_g2s(smem_u32(sh->rows + t * kHidStride), a.hidden + (size_t)t * kHidden, kHidden, hb);
-        if (blockIdx.x == 0) ws.ctrl->dec_phase = 0;   // second barrier's counter, see grid_barrier
+            bulk_g2s(smem_u32(sh->pool + t * kHidStride), a.hidden + (size_t)t * kHidden, kHidden, hb);
     }
     for (int q = tid; q < T * kHiddenBlocks; q += kDecThreads) {
         const int t = q % T, kb = q / T;
@@ -205,17 +247,17 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
     }
 
     // ------------------------------------------------------------------ routing (every CTA)
-    // For one or two tokens: the same selection as route_token_warp (route_token.cuh), spread over
-    // the CTA's 16 warps, because the single-warp routine's chain of dependent reductions (about
-    // 4 us) would be the longest serial stretch of the kernel.  Scores and their order-preserving keys go to
+    // For up to three tokens: the same selection as route_token_warp (route_token.cuh), spread over the CTA's
+    // warps (2.6 us for one token, 1.1 us more for each further one, where a warp per token takes 5 us for any
+    // number of them).  Scores and their order-preserving keys go to
     // shared memory; one warp per (token, group) forms the group score; one thread per token keeps
     // the four best groups; then the eight argmax rounds are replaced by counting, for each of the
     // 128 live scores, how many of the others beat it (higher key, or equal key and earlier in the
     // reference's tie order): the score with count k is the k-th pick.  Same picks, same order.
-    if (tid < kMaxLocalExperts) sh->expert_slot[tid] = -1;
-    float* r_s = reinterpret_cast<float*>(&sh->wring[1][kRing - 1][0]);                 // [T][256], idle ring slot
+    if (tid < kMaxLocalExperts) sh->expert_m[tid] = 0;
+    if (tid < kDecMaxActive) sh->pair_le[tid] = -1;
+    float* r_s = reinterpret_cast<float*>(sh->pool + rows_tokens(T) * kHidStride);        // [T][256], idle ring
     uint32_t* r_key = reinterpret_cast<uint32_t*>(r_s + kDecodeMaxTokens * kNumExperts);  // [T][256]
-    static_assert(2 * kDecodeMaxTokens * kNumExperts * 4 <= kStepRows * kStepStride, "routing scratch fits a ring slot");
     stamp(12);
     if (T <= kCoopRouteTokens) {
         for (int q = tid; q < T * kNumExperts; q += kDecThreads) {
@@ -226,7 +268,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
         }
         for (int q = tid; q < T * kTopKGroup * 32; q += kDecThreads) (&sh->r_count[0][0][0])[q] = 0;
         __syncthreads();
-        for (int task = warp; task < T * kNumGroups; task += kDecWarps) {   // group score = two largest of the group
+        for (int task = warp; task < T * kNumGroups; task += kDecThreads / 32) {   // group score = two largest of the group
             const uint32_t key = r_key[task * 32 + lane];
             const uint32_t k1 = __reduce_max_sync(0xffffffffu, key);
             const uint32_t holders = __ballot_sync(0xffffffffu, key == k1);
@@ -240,6 +282,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
             for (int k = 0; k < kTopKGroup; ++k) {
                 float best = kNegSentinel;
                 int best_i = -1;
+#pragma unroll
                 for (int i = 0; i < kNumGroups; ++i) {
                     const float gsc = sh->r_gscore[tid][i];
                     if (!((kept_mask >> i) & 1u) && gsc > best) { best = gsc; best_i = i; }
@@ -255,14 +298,14 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
         __syncthreads();
         // count[t][j][lane]: how many live scores beat score `lane` of the j-th kept group; the work of one
         // (token, group) is split over four warps, one per opposing group
-        for (int task = warp; task < T * kTopKGroup * kTopKGroup; task += kDecWarps) {
+        for (int task = warp; task < T * kTopKGroup * kTopKGroup; task += kDecThreads / 32) {
             const int t = task / (kTopKGroup * kTopKGroup), j = (task / kTopKGroup) % kTopKGroup, part = task % kTopKGroup;
             const int g = sh->r_kept[t][j], g2 = sh->r_kept[t][part];
             const uint32_t key = r_key[t * kNumExperts + g * 32 + lane];
             const uint32_t tie = (uint32_t)g * 32u + (__brev((uint32_t)lane) >> 27);
             const uint32_t* other = r_key + t * kNumExperts + g2 * 32;
             int beat = 0;
-    #pragma unroll 8
+#pragma unroll 8
             for (int l2 = 0; l2 < 32; ++l2) {
                 const uint32_t key2 = other[l2];
                 const uint32_t tie2 = (uint32_t)g2 * 32u + (__brev((uint32_t)l2) >> 27);
@@ -271,7 +314,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
             atomicAdd(&sh->r_count[t][j][lane], beat);
         }
         __syncthreads();
-        for (int task = warp; task < T * kTopKGroup; task += kDecWarps) {
+        for (int task = warp; task < T * kTopKGroup; task += kDecThreads / 32) {
             const int t = task / kTopKGroup, j = task % kTopKGroup;
             const int rank = sh->r_count[t][j][lane];
             if (rank < kTopK) {
@@ -280,26 +323,21 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
                 sh->r_sel[t][rank] = r_s[t * kNumExperts + ge];
             }
         }
-        __syncthreads();
     } else if (warp < T) {
         // more tokens than that: one warp per token runs the staged chain's routine, the tokens in parallel
         int idx[kTopK];
         float wn[kTopK];
         route_token_warp(a.logits + (size_t)warp * kNumExperts, a.bias, lane, idx, wn);
-        if (lane < kTopK) {
-            int my_idx = 0;
-            float my_s = 0.0f;
 #pragma unroll
-            for (int k = 0; k < kTopK; ++k)
-                if (k == lane) { my_idx = idx[k]; my_s = wn[k]; }
-            sh->r_idx[warp][lane] = my_idx;
-            sh->r_sel[warp][lane] = my_s;   // already normalised
-        }
+        for (int k = 0; k < kTopK; ++k)
+            if (k == lane) { sh->r_idx[warp][k] = idx[k]; sh->r_sel[warp][k] = wn[k]; }   // already normalised
     }
-    if (T > kCoopRouteTokens) __syncthreads();
+    __syncthreads();
     stamp(8);
-    if (tid < T) {
-        const int t = tid;
+    // Dispatch, one warp per token: lane s applies the policy to 32-expert shard s, and a lane's pairs follow
+    // those of the lanes before it.
+    if (warp < T) {
+        const int t = warp;
         int idx[kTopK];
         float wn[kTopK];
         float sumw = 1e-20f;
@@ -308,186 +346,280 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
         const float inv = 1.0f / sumw;
 #pragma unroll
         for (int k = 0; k < kTopK; ++k) wn[k] = T <= kCoopRouteTokens ? sh->r_sel[t][k] * inv : sh->r_sel[t][k];
-        if (blockIdx.x == 0) {
-#pragma unroll
-            for (int k = 0; k < kTopK; ++k) {
-                ws.topk_idx[(size_t)t * kTopK + k] = idx[k];
-                ws.topk_weight[(size_t)t * kTopK + k] = wn[k];
-            }
+        if (blockIdx.x == 0 && lane < kTopK) {
+            ws.topk_idx[(size_t)t * kTopK + lane] = sh->r_idx[t][lane];
+            ws.topk_weight[(size_t)t * kTopK + lane] = T <= kCoopRouteTokens ? sh->r_sel[t][lane] * inv : sh->r_sel[t][lane];
         }
         int n_pairs = 0;
         int p_le[kTopK];
         float p_w[kTopK];
 #pragma unroll
         for (int i = 0; i < kTopK; ++i) { p_le[i] = 0; p_w[i] = 0.0f; }
-        const int shards = E / kShardExperts;
-        for (int sdx = 0; sdx < shards; ++sdx)
-            dispatch_one_shard(idx, wn, sdx, a.local_expert_offset, a.pol, a.rsf, n_pairs, p_le, p_w);
-        sh->pair_count[t] = n_pairs;
+        if (lane < E / kShardExperts) dispatch_one_shard(idx, wn, lane, a.local_expert_offset, a.pol, a.rsf, n_pairs, p_le, p_w);
+        int incl = n_pairs;
 #pragma unroll
-        for (int i = 0; i < kTopK; ++i) { sh->pair_le[t][i] = p_le[i]; sh->pair_w[t][i] = p_w[i]; }
+        for (int off = 1; off < 8; off <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += y;
+        }
+        const int pair_base = incl - n_pairs;
+#pragma unroll
+        for (int i = 0; i < kTopK; ++i) {
+            if (i < n_pairs) {
+                sh->pair_le[t * kTopK + pair_base + i] = p_le[i];
+                sh->pair_w[t * kTopK + pair_base + i] = p_w[i];
+            }
+        }
+        if (lane == 7) sh->pair_count[t] = incl;
         stamp(9);
     }
     __syncthreads();
-    if (tid == 0) {
-        // active experts in order of first use, rows of an expert in token order: the same in
-        // every CTA, so unit u means the same thing everywhere
-        int n_active = 0;
-        for (int t = 0; t < T; ++t) {
-            const int np = sh->pair_count[t];
-            for (int p = 0; p < np; ++p) {
-                const int le = sh->pair_le[t][p];
-                int ai = sh->expert_slot[le];
-                if (ai < 0) {
-                    ai = n_active++;
-                    sh->expert_slot[le] = ai;
-                    sh->act_expert[ai] = le;
-                    sh->act_m[ai] = 0;
-                }
-                const int slot = sh->act_m[ai]++;
-                sh->act_tok[ai][slot] = t;
-                sh->pair_slot[t][p] = slot;
+    // Active experts in order of first use, rows of an expert in token order: the same in every CTA, so unit u
+    // means the same thing everywhere.  One thread per (token, pair) entry looks the others over.
+    const int n_entries = T * kTopK;
+    const int my_le = tid < n_entries ? sh->pair_le[tid] : -1;
+    int my_first = kDecMaxActive, my_slot = 0, my_m = 0;
+    if (my_le >= 0) {
+        for (int j = 0; j < n_entries; ++j) {
+            if (sh->pair_le[j] == my_le) {
+                ++my_m;
+                if (j < tid) ++my_slot;
+                if (my_first == kDecMaxActive) my_first = j;
             }
         }
-        int rows = 0;
-        for (int ai = 0; ai < n_active; ++ai) { sh->act_row0[ai] = rows; rows += sh->act_m[ai]; }
-        sh->n_active = n_active;
-        sh->n_rows = rows;
-        stamp(10);
     }
+    if (tid < n_entries) sh->pair_first[tid] = my_first;
+    const int n_active = __syncthreads_count(my_le >= 0 && my_first == tid);
+    if (my_le >= 0) {
+        int ai = 0, row0 = 0;
+        for (int j = 0; j < n_entries; ++j) {
+            const int f = sh->pair_first[j];
+            if (f < my_first) { ++row0; ai += f == j ? 1 : 0; }
+        }
+        if (my_first == tid) {
+            sh->act_expert[ai] = my_le;
+            sh->act_m[ai] = my_m;
+            sh->act_row0[ai] = row0;
+            sh->expert_m[my_le] = my_m;
+        }
+        sh->act_tok[ai][my_slot] = tid / kTopK;
+        if (blockIdx.x == 0) {   // the tables that the combine, other entry points and the tests read
+            ws.pair_code[tid] = ((uint32_t)my_le << 24) | (uint32_t)my_slot;
+            ws.pair_weight[tid] = sh->pair_w[tid];
+        }
+        if (blockIdx.x == 0) ws.pair_row[tid] = row0 + my_slot;
+    } else if (blockIdx.x == 0 && tid < n_entries) {
+        ws.pair_row[tid] = -1;
+    }
+    if (blockIdx.x == 0 && tid < T) ws.pair_count[tid] = sh->pair_count[tid];
+    stamp(10);
     __syncthreads();
-    if (tid < T * kTopK) {
-        const int t = tid / kTopK, p = tid % kTopK;
-        if (p < sh->pair_count[t]) sh->pair_row[t][p] = sh->act_row0[sh->expert_slot[sh->pair_le[t][p]]] + sh->pair_slot[t][p];
-    }
-    if (blockIdx.x == 0) {   // the tables other entry points and the tests read
-        if (tid < T) ws.pair_count[tid] = sh->pair_count[tid];
-        if (tid < T * kTopK) {
-            const int t = tid / kTopK, p = tid % kTopK;
-            if (p < sh->pair_count[t]) {
-                ws.pair_code[tid] = ((uint32_t)sh->pair_le[t][p] << 24) | (uint32_t)sh->pair_slot[t][p];
-                ws.pair_weight[tid] = sh->pair_w[t][p];
-            }
-        }
-        if (tid < E) {
-            const int ai = sh->expert_slot[tid];
-            ws.ctrl->expert_rows[tid] = ai >= 0 ? sh->act_m[ai] : 0;
-        }
-    }
+    if (blockIdx.x == 0 && tid < E) ws.ctrl->expert_rows[tid] = sh->expert_m[tid];
     stamp(11);
-    __syncthreads();
-    const int n_active = sh->n_active;
     stamp(1);
-    float* act = ws.splitk_partial;   // [rows, 2048] fp32 SwiGLU output (the split-K scratch is idle on this path)
+    float* act = ws.dec_act;   // [rows, 2048] fp32 SwiGLU output
 
-    // The 16 warps work as two independent halves of 8 (named barriers 1 and 2): a half is one
-    // worker with its own unit range, weight ring and reduction buffer, so an SM always has two
-    // units in flight and the unit ranges are twice as fine.  Thread 0 of a half is its producer:
-    // it issues the bulk copies of a step (16 rows x 1 KB) as soon as the ring slot is free -- of
-    // the next unit and, before the grid barrier, of the next phase as well.  Warp hw of the half
-    // consumes K block hw of every step.
-    const int half = warp >> 3, hw = warp & (kHalfWarps - 1), htid = tid & (kHalfThreads - 1);
-    const int workers = (int)gridDim.x * 2, wk = (int)blockIdx.x * 2 + half;
+    // The 16 consumer warps work as two independent halves of 8 (named barriers 1 and 2): a half is one
+    // worker with its own weight ring and reduction buffer, so an SM always has two
+    // units in flight and the work is dealt twice as finely.  A producer warp per half (one lane) draws the units
+    // and requests a step (16 rows x 1 KB) as soon as its ring slot is free -- of the next unit and of the next
+    // phase as well.  Warp hw of the half consumes K block hw of every step.
+    const bool producer = warp >= kDecWarps;
+    const int half = producer ? warp - kDecWarps : warp >> 3, hw = warp & (kHalfWarps - 1), htid = tid & (kHalfThreads - 1);
+    const int workers = (int)gridDim.x * 2;
     const int bar_id = 1 + half;
-    const bool producer = htid == 0;
-    const int units1 = n_active * kG1Units, units2 = n_active * kG2Units;
-    const int u1_begin = (int)((long long)units1 * wk / workers), u1_end = (int)((long long)units1 * (wk + 1) / workers);
-    const int u2_begin = (int)((long long)units2 * wk / workers), u2_end = (int)((long long)units2 * (wk + 1) / workers);
-    const int S1 = (u1_end - u1_begin) * kG1Steps, S2 = (u2_end - u2_begin) * kG2Steps;
-    int issued = 0;     // steps issued so far by this half's producer (both phases)
-    int consumed = 0;   // steps consumed so far by this half
-    bool ok = true;
-
-    // producer only: step s of phase 1 (s < S1) or phase 2 (s - S1)
-    auto issue = [&](int s) -> bool {
-        const int slot = issued & (kRing - 1);
-        if (issued >= kRing &&
-            !mbar_wait(smem_u32(&sh->empty_bar[half][slot]), (uint32_t)((issued / kRing - 1) & 1), abort_flag))
-            return false;
-        const uint32_t bar = smem_u32(&sh->full_bar[half][slot]);
-        const uint32_t dst = smem_u32(&sh->wring[half][slot][0]);
-        mbar_expect_tx(bar, kStepBytes);
-        if (s < S1) {
-            const int u = u1_begin + s / kG1Steps, i = s % kG1Steps;
-            const int row = sh->act_expert[u / kG1Units] * kGemm1Out + (u % kG1Units) * kG1Cols;
-            tma_load_2d(dst, &tmap_w1, bar, i * (kStepK / 4), row);                              // 8 linear rows
-            tma_load_2d(dst + 8 * kStepStride, &tmap_w1, bar, i * (kStepK / 4), row + kInter);   // 8 gated rows
-        } else {
-            const int s2 = s - S1;
-            const int u = u2_begin + s2 / kG2Steps, i = s2 % kG2Steps;
-            tma_load_2d(dst, &tmap_w2, bar, i * (kStepK / 4), sh->act_expert[u / kG2Units] * kHidden + (u % kG2Units) * kG2Cols);
-        }
-        ++issued;
-        return true;
-    };
-    // everybody: wait for the next step's bytes; returns the ring slot
-    auto acquire = [&]() -> const uint8_t* {
-        const int slot = consumed & (kRing - 1);
-        if (!mbar_wait(smem_u32(&sh->full_bar[half][slot]), (uint32_t)((consumed / kRing) & 1), abort_flag)) ok = false;
-        return &sh->wring[half][slot][0];
-    };
-    auto release = [&]() {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sh->empty_bar[half][consumed & (kRing - 1)]));
-        ++consumed;
-    };
+    const int ring = T <= kFewTokens ? kRingFew : kRing;
+    uint8_t* const wring = sh->pool + rows_tokens(T) * kHidStride + half * ring * kStepBytes;
+    uint64_t* const full_bar = sh->full_bar[half];
+    uint64_t* const empty_bar = sh->empty_bar[half];
 
     if (producer) {
-        for (int s = 0; s < kRing && s < S1 + S2 && ok; ++s)
-            if (s < S1 || S1 == 0) ok = issue(s);   // phase-2 steps are not issued ahead of phase 1 here, see below
+        if (lane != 0) return;
+        PhasePlan p1, p2;
+        p1.make(n_active * kG1Units, workers);
+        p2.make(n_active * kG2Units, workers);
+        const int tickets = p1.tickets + p2.tickets;
+        int slot = 0, issued = 0;
+        uint32_t phase = 1;   // the first pass over the ring finds every slot free
+        bool ok = true;
+        auto range_of = [&](int ticket, int& begin, int& end, int& bit) {
+            if (ticket < p1.tickets) { p1.range(ticket, begin, end); bit = 0; }
+            else { p2.range(ticket - p1.tickets, begin, end); bit = kPhase2Bit; }
+        };
+        int ticket = n_active > 0 ? (int)atomicAdd(&ws.ctrl->dec_ticket, 1u) : tickets;
+        while (ok && ticket < tickets) {
+            int u, end, bit;
+            range_of(ticket, u, end, bit);
+            int next_ticket = tickets;
+            for (; ok && u < end; ++u) {
+                const int steps = bit ? kG2Steps : kG1Steps;
+                const int ai = bit ? u / kG2Units : u / kG1Units;
+                const int in = bit ? u - ai * kG2Units : u - ai * kG1Units;
+                const int row = bit ? sh->act_expert[ai] * kHidden + in * kG2Cols : sh->act_expert[ai] * kGemm1Out + in * kG1Cols;
+                // The next ticket is drawn with the run's last unit: early enough for its round trip to pass while
+                // that unit's steps are requested, and not before (a ticket drawn with a long run still ahead
+                // would be held for that long).
+                if (u + 1 == end) next_ticket = (int)atomicAdd(&ws.ctrl->dec_ticket, 1u);
+                for (int i = 0; i < steps; ++i) {
+                    if (!mbar_wait(smem_u32(&empty_bar[slot]), phase, abort_flag)) { ok = false; break; }
+                    int next = u + 1 < end ? u + 1 + bit : -1;
+                    if (u + 1 == end && i >= (steps > 2 ? 2 : steps - 1) && next_ticket < tickets) {
+                        // by now the next ticket is there: the run's last unit names the first of the next run
+                        int nb, ne, nbit;
+                        range_of(next_ticket, nb, ne, nbit);
+                        next = nb + nbit;
+                    }
+                    sh->step_desc[half][slot] = make_int4(u + bit, i, next, 0);
+                    const uint32_t bar = smem_u32(&full_bar[slot]);
+                    const uint32_t dst = smem_u32(wring + slot * kStepBytes);
+                    mbar_expect_tx(bar, kStepBytes);
+                    if (!bit) {
+                        tma_load_2d(dst, &tmap_w1, bar, i * (kStepK / 4), row);                              // 8 linear rows
+                        tma_load_2d(dst + 8 * kStepStride, &tmap_w1, bar, i * (kStepK / 4), row + kInter);   // 8 gated rows
+                    } else {
+                        tma_load_2d(dst, &tmap_w2, bar, i * (kStepK / 4), row);
+                    }
+                    ++issued;
+                    if (++slot == ring) { slot = 0; phase ^= 1u; }
+                }
+            }
+            ticket = next_ticket;
+        }
+        if (ok && mbar_wait(smem_u32(&empty_bar[slot]), phase, abort_flag)) {
+            sh->step_desc[half][slot] = make_int4(-1, 0, -1, 0);
+            mbar_arrive(smem_u32(&full_bar[slot]));
+        } else {
+            // leave only after the copies in flight have landed (bounded)
+            for (int g = issued > ring ? issued - ring : 0; g < issued; ++g) {
+                const uint32_t bar = smem_u32(&full_bar[g % ring]);
+                const uint64_t t0 = global_timer_ns();
+                while (!mbar_try_wait(bar, (uint32_t)((g / ring) & 1)) && global_timer_ns() - t0 < kWaitLimitNs) {}
+            }
+        }
+        return;
     }
+
+    int slot = 0;            // ring slot and parity of the next step to consume
+    uint32_t phase = 0;
+    bool ok = true;
+    auto release = [&]() {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&empty_bar[slot]));
+        if (++slot == ring) { slot = 0; phase ^= 1u; }
+    };
+    // The weight scales of a unit's K blocks sit in lanes of the warp that uses them (phase 1: lanes 0..13, 7
+    // linear and 7 gated; phase 2: lanes 0 and 1), fetched one unit ahead so that no step waits for them.
+    auto unit_scales = [&](int unit) -> float {
+        float v = 0.0f;
+        if (unit & kPhase2Bit) {
+            const int u = unit - kPhase2Bit;
+            if (lane < kG2Steps) {
+                const int e = sh->act_expert[u / kG2Units], hh = u % kG2Units;
+                v = __ldg(a.s2 + ((size_t)e * kHiddenBlocks + hh / (kBlock / kG2Cols)) * kInterBlocks + hw + kHalfWarps * lane);
+            }
+        } else if (lane < 2 * kG1Steps) {
+            const int e = sh->act_expert[unit / kG1Units], gg = unit % kG1Units;
+            const int blk = gg / (kBlock / kG1Cols) + (lane >= kG1Steps ? kInter / kBlock : 0);
+            const int kb = hw + kHalfWarps * (lane % kG1Steps);
+            v = __ldg(a.s1 + ((size_t)e * (kGemm1Out / kBlock) + blk) * kHiddenBlocks + kb);
+        }
+        return v;
+    };
     // the hidden rows must have landed before the first MMA
     if (!mbar_wait(smem_u32(&sh->hid_bar), 0u, abort_flag)) ok = false;
 
-    // ------------------------------------------------------------------ phase 1: GEMM1 + SwiGLU
-    {
-        int ai = 0, g = 0, m = 0;
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        // The weight scales of a unit's K blocks sit in lanes 0..13 of the warp that uses them (7
-        // linear, 7 gated), fetched one unit ahead so that no step waits for them.
-        auto unit_scales = [&](int u) -> float {
-            float v = 0.0f;
-            if (u < u1_end && lane < 2 * kG1Steps) {
-                const int e = sh->act_expert[u / kG1Units], gg = u % kG1Units;
-                const int blk = gg / (kBlock / kG1Cols) + (lane >= kG1Steps ? kInter / kBlock : 0);
-                const int kb = hw + kHalfWarps * (lane % kG1Steps);
-                v = __ldg(a.s1 + ((size_t)e * (kGemm1Out / kBlock) + blk) * kHiddenBlocks + kb);
+    uint8_t* a2rows = sh->pool + half * (rows_tokens(T) * kA2Stride);
+    float(*a2s)[kInterBlocks] = sh->a2_scale[half];
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float sc_cur = 0.0f, sc_next = 0.0f;
+    int ai = 0, in = 0, m = 0, staged = -1, parity = 0;
+    int loaded_for = -1;   // unit that sc_next belongs to
+    bool in_phase2 = false;
+    while (ok) {
+        if (!mbar_wait(smem_u32(&full_bar[slot]), phase, abort_flag)) { ok = false; break; }
+        const int4 d = sh->step_desc[half][slot];
+        if (d.x < 0) break;
+        const uint8_t* wst = wring + slot * kStepBytes;
+        const int i = d.y;
+        const bool p2 = (d.x & kPhase2Bit) != 0;
+        if (i == 0) {   // a new unit
+            const int u = p2 ? d.x - kPhase2Bit : d.x;
+            ai = p2 ? u / kG2Units : u / kG1Units;
+            in = p2 ? u - ai * kG2Units : u - ai * kG1Units;
+            m = sh->act_m[ai];
+            sc_cur = loaded_for == d.x ? sc_next : unit_scales(d.x);
+            acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
+            if (p2 && ai != staged) {
+                // ---------------------------------------------------- another expert's rows for phase 2
+                if (!in_phase2) {
+                    // the hidden rows are overwritten below: both halves have to be through with them
+                    stamp(2);
+                    named_bar_sync(3, kConsumers);
+                    in_phase2 = true;
+                }
+                named_bar_sync(bar_id, kHalfThreads);   // the half is done with the previous expert's rows
+                if (staged < 0) stamp(3);
+                // 1x128 requantisation of the expert's rows, as in the staged GEMM1 epilogue:
+                // scale = amax / 448 (1 if the block is zero), payload e4m3(v * (1 / scale))
+                for (int item = hw; item < m * kInterBlocks; item += kHalfWarps) {
+                    const int row = item / kInterBlocks, ib = item % kInterBlocks;
+                    const float* src = act + (size_t)(sh->act_row0[ai] + row) * kInter + ib * kBlock + lane * 4;
+                    float4 v = ld_relaxed_gpu(src);
+                    if (!__all_sync(0xffffffffu, is_there(v))) {   // phase-1 units of other workers still under way
+                        const uint64_t t0 = global_timer_ns();
+                        do {
+                            if (!is_there(v)) v = ld_relaxed_gpu(src);
+                            if (*abort_flag != 0 || global_timer_ns() - t0 > kWaitLimitNs) sh->abort = 1;
+                        } while (!__all_sync(0xffffffffu, is_there(v) || *abort_flag != 0));
+                    }
+                    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                    const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
+                    const float inv = 1.0f / sc;
+                    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v.x * inv, v.y * inv), __NV_SATFINITE, __NV_E4M3);
+                    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v.z * inv, v.w * inv), __NV_SATFINITE, __NV_E4M3);
+                    *reinterpret_cast<uint32_t*>(a2rows + row * kA2Stride + ib * kBlock + lane * 4) = lo | (hi << 16);
+                    if (lane == 0) a2s[row][ib] = sc;
+                }
+                named_bar_sync(bar_id, kHalfThreads);
+                if (*abort_flag != 0) { ok = false; break; }
+                staged = ai;
             }
-            return v;
-        };
-        float sc_cur = 0.0f, sc_next = unit_scales(u1_begin);
-        for (int s = 0; s < S1 && ok; ++s) {
-            const int u = u1_begin + s / kG1Steps, i = s % kG1Steps;
-            if (i == 0) {   // a new unit
-                ai = u / kG1Units;
-                g = u % kG1Units;
-                m = sh->act_m[ai];
-                sc_cur = sc_next;
-                sc_next = unit_scales(u + 1);
-                acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
-            }
-            const int kb = hw + kHalfWarps * i;
+        }
+        const int kb = hw + kHalfWarps * i;
+        float raw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (!p2) {
+            // -------------------------------------------------------- phase 1: GEMM1 + SwiGLU
             const float sl = __shfl_sync(0xffffffffu, sc_cur, i), sg = __shfl_sync(0xffffffffu, sc_cur, kG1Steps + i);
             const int tok = sh->act_tok[ai][r < m ? r : 0];
-            const uint8_t* wst = acquire();
-            if (!ok) break;
-            float raw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            mma_block(raw, wst + r * kStepStride + hw * kBlock + 16 * c, sh->rows + tok * kHidStride + kb * kBlock + 16 * c);
+            mma_block(raw, wst + r * kStepStride + hw * kBlock + 16 * c, sh->pool + tok * kHidStride + kb * kBlock + 16 * c);
             release();
-            if (producer && s + kRing < S1 + S2) {
-                // phase-2 steps may be issued from here on: their slots were phase-1 slots that are now free
-                if (!issue(s + kRing)) { ok = false; }
-            }
             const int t0 = sh->act_tok[ai][2 * c < m ? 2 * c : 0], t1 = sh->act_tok[ai][2 * c + 1 < m ? 2 * c + 1 : 0];
             const float sa0 = sh->hid_scale[t0][kb], sa1 = sh->hid_scale[t1][kb];
             acc[0] = fmaf(raw[0], sa0 * sl, acc[0]);
             acc[1] = fmaf(raw[1], sa1 * sl, acc[1]);
             acc[2] = fmaf(raw[2], sa0 * sg, acc[2]);
             acc[3] = fmaf(raw[3], sa1 * sg, acc[3]);
-            if (i == kG1Steps - 1) {   // the unit is complete: add the eight warps' partial sums
-                float* red = &sh->red[half][u & 1][0][0];
-                *reinterpret_cast<float4*>(red + hw * 128 + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                named_bar_sync(bar_id, kHalfThreads);
+        } else {
+            // -------------------------------------------------------- phase 2: GEMM2
+            const float sw = __shfl_sync(0xffffffffu, sc_cur, i);
+            mma_block(raw, wst + r * kStepStride + hw * kBlock + 16 * c, a2rows + r * kA2Stride + kb * kBlock + 16 * c);
+            release();
+            const float sa0 = a2s[2 * c][kb] * sw, sa1 = a2s[2 * c + 1][kb] * sw;
+            acc[0] = fmaf(raw[0], sa0, acc[0]);
+            acc[1] = fmaf(raw[1], sa1, acc[1]);
+            acc[2] = fmaf(raw[2], sa0, acc[2]);
+            acc[3] = fmaf(raw[3], sa1, acc[3]);
+        }
+        const bool last = i == (p2 ? kG2Steps : kG1Steps) - 1;
+        if (d.z >= 0 && d.z != loaded_for) { sc_next = unit_scales(d.z); loaded_for = d.z; }
+        if (last) {   // the unit is complete: add the eight warps' partial sums
+            float* red = &sh->red[half][parity][0][0];
+            parity ^= 1;
+            *reinterpret_cast<float4*>(red + hw * 128 + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            named_bar_sync(bar_id, kHalfThreads);
+            if (!p2) {
                 if (htid < 64) {
                     const int l = htid & 31, jj = htid >> 5;
                     float lin = 0.0f, gate = 0.0f;
@@ -496,151 +628,90 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
                         lin += red[w * 128 + l * 4 + jj];
                         gate += red[w * 128 + l * 4 + 2 + jj];
                     }
-                    const int slot = 2 * (l & 3) + jj, col = g * kG1Cols + (l >> 2);
-                    if (slot < m) {
+                    const int row = 2 * (l & 3) + jj, col = in * kG1Cols + (l >> 2);
+                    if (row < m) {
                         const float x1 = round_bf16(lin), x2 = round_bf16(gate);
                         const float silu = a.silu_exact ? x2 / (1.0f + __expf(-x2))
                                                         : x2 * (0.5f * (x2 * rsqrtf(fmaf(x2, x2, 4.0f)) + 1.0f));
-                        act[(size_t)(sh->act_row0[ai] + slot) * kInter + col] = silu * x1;
+                        st_relaxed_gpu(act + (size_t)(sh->act_row0[ai] + row) * kInter + col, silu * x1);
                     }
                 }
+            } else if (htid < 128) {
+                const int l = htid >> 2, q = htid & 3;
+                const int row = 2 * (l & 3) + (q & 1), hrow = in * kG2Cols + (l >> 2) + 8 * (q >> 1);
+                float sum = 0.0f;
+#pragma unroll
+                for (int w = 0; w < kHalfWarps; ++w) sum += red[w * 128 + l * 4 + q];
+                if (row < m) ws.y[(size_t)(sh->act_row0[ai] + row) * kHidden + hrow] = __float2bfloat16_rn(sum);
             }
         }
     }
-    if (producer && S1 == 0 && ok) {   // nothing to do in phase 1: start phase 2's first steps now
-        for (int s = issued; s < kRing && s < S2 && ok; ++s) ok = issue(s);
+    if (!in_phase2) {   // the other half may be waiting to overwrite the hidden rows
+        stamp(2);
+        named_bar_sync(3, kConsumers);
+        stamp(3);
     }
-
-    // A half that gave up on a wait still lets its bulk copies land before the CTA may exit.
-    auto give_up = [&]() {
+    if (!ok) {
+        // a half that gave up on a wait says so; the producers let their copies land before they leave
         atomicCAS(&ws.ctrl->status, kStatusOk, kStatusDecodeTimeout);
         sh->abort = 1;
-        if (producer) {
-            for (int g = consumed; g < issued; ++g) {
-                const uint32_t bar = smem_u32(&sh->full_bar[half][g & (kRing - 1)]);
-                const uint64_t t0 = global_timer_ns();
-                while (!mbar_try_wait(bar, (uint32_t)((g / kRing) & 1)) && global_timer_ns() - t0 < kWaitLimitNs) {}
-            }
-        }
-    };
-
-    // ------------------------------------------------------------------ phase 2: requant + GEMM2
-    stamp(2);
-    if (!ok) give_up();
-    if (!grid_barrier(&ws.ctrl->dec_count, ws.ctrl, sh)) {
-        if (ok) give_up();
-        return;
     }
-    stamp(3);
-    {
-        uint8_t* a2rows = sh->rows + half * (kDecodeMaxTokens * kA2Stride);
-        float(*a2s)[kInterBlocks] = sh->a2_scale[half];
-        int staged = -1, ai = 0, hg = 0, m = 0;
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        auto unit_scales2 = [&](int u) -> float {   // lanes 0 and 1: this warp's two K blocks, one unit ahead
-            float v = 0.0f;
-            if (u < u2_end && lane < kG2Steps) {
-                const int e = sh->act_expert[u / kG2Units], hh = u % kG2Units;
-                v = __ldg(a.s2 + ((size_t)e * kHiddenBlocks + hh / (kBlock / kG2Cols)) * kInterBlocks + hw + kHalfWarps * lane);
-            }
-            return v;
-        };
-        float sc_cur = 0.0f, sc_next = unit_scales2(u2_begin);
-        for (int s = 0; s < S2 && ok; ++s) {
-            const int u = u2_begin + s / kG2Steps, i = s % kG2Steps;
-            if (i == 0) {
-                ai = u / kG2Units;
-                hg = u % kG2Units;
-                m = sh->act_m[ai];
-                if (ai != staged) {
-                    named_bar_sync(bar_id, kHalfThreads);   // the half is done with the previous expert's rows
-                    // 1x128 requantisation of the expert's rows, as in the staged GEMM1 epilogue:
-                    // scale = amax / 448 (1 if the block is zero), payload e4m3(v * (1 / scale))
-                    for (int item = hw; item < m * kInterBlocks; item += kHalfWarps) {
-                        const int slot = item / kInterBlocks, ib = item % kInterBlocks;
-                        const float4 v = __ldcg(reinterpret_cast<const float4*>(
-                            act + (size_t)(sh->act_row0[ai] + slot) * kInter + ib * kBlock) + lane);
-                        float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                        const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
-                        const float inv = 1.0f / sc;
-                        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v.x * inv, v.y * inv), __NV_SATFINITE, __NV_E4M3);
-                        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v.z * inv, v.w * inv), __NV_SATFINITE, __NV_E4M3);
-                        *reinterpret_cast<uint32_t*>(a2rows + slot * kA2Stride + ib * kBlock + lane * 4) = lo | (hi << 16);
-                        if (lane == 0) a2s[slot][ib] = sc;
-                    }
-                    named_bar_sync(bar_id, kHalfThreads);
-                    staged = ai;
-                }
-                sc_cur = sc_next;
-                sc_next = unit_scales2(u + 1);
-                acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
-            }
-            const int kb = hw + kHalfWarps * i;
-            const float sw = __shfl_sync(0xffffffffu, sc_cur, i);
-            const uint8_t* wst = acquire();
-            if (!ok) break;
-            float raw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            mma_block(raw, wst + r * kStepStride + hw * kBlock + 16 * c, a2rows + r * kA2Stride + kb * kBlock + 16 * c);
-            release();
-            if (producer && s + kRing < S2) {
-                if (!issue(S1 + s + kRing)) { ok = false; }
-            }
-            const float sa0 = a2s[2 * c][kb] * sw, sa1 = a2s[2 * c + 1][kb] * sw;
-            acc[0] = fmaf(raw[0], sa0, acc[0]);
-            acc[1] = fmaf(raw[1], sa1, acc[1]);
-            acc[2] = fmaf(raw[2], sa0, acc[2]);
-            acc[3] = fmaf(raw[3], sa1, acc[3]);
-            if (i == kG2Steps - 1) {
-                float* red = &sh->red[half][u & 1][0][0];
-                *reinterpret_cast<float4*>(red + hw * 128 + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                named_bar_sync(bar_id, kHalfThreads);
-                if (htid < 128) {
-                    const int l = htid >> 2, q = htid & 3;
-                    const int slot = 2 * (l & 3) + (q & 1), hrow = hg * kG2Cols + (l >> 2) + 8 * (q >> 1);
-                    float sum = 0.0f;
-#pragma unroll
-                    for (int w = 0; w < kHalfWarps; ++w) sum += red[w * 128 + l * 4 + q];
-                    if (slot < m) ws.y[(size_t)(sh->act_row0[ai] + slot) * kHidden + hrow] = __float2bfloat16_rn(sum);
-                }
-            }
-        }
-    }
-    if (!ok) give_up();
-
-    // ------------------------------------------------------------------ phase 3: weighted combine
     stamp(4);
-    if (!grid_barrier(&ws.ctrl->dec_phase, ws.ctrl, sh)) return;
-    if (blockIdx.x == 0 && tid == 0) ws.ctrl->dec_count = 0;   // everybody has left the first barrier
-    stamp(5);
-    {
-        constexpr int kChunks = kHidden / 8;   // 16-byte chunks of a row
-        for (int i = blockIdx.x * kDecThreads + tid; i < T * kChunks; i += gridDim.x * kDecThreads) {
-            const int t = i / kChunks, ch = i % kChunks;
-            float acc[8];
+}
+
+// The weighted combine of the decode kernel's rows: same arithmetic and pair order as combine_kernel, the rows
+// found through pair_row (one load instead of pair code -> expert offset), all requested at once.  Small CTAs
+// (a seventh of a row each), so that they fit beside a running decode CTA's registers.
+constexpr int kDecCombineThreads = 128;
+constexpr int kDecCombineParts = kHidden / 8 / kDecCombineThreads;   // 7
+static_assert(kDecCombineParts * kDecCombineThreads * 8 == kHidden, "a row splits into whole CTAs");
+__global__ void __launch_bounds__(kDecCombineThreads) decode_combine_kernel(Workspace ws, __nv_bfloat16* __restrict__ out)
+{
+    const int t = blockIdx.y, ch = blockIdx.x * kDecCombineThreads + threadIdx.x;
+    const bool clocked = t == 0 && blockIdx.x == 0 && threadIdx.x == 0;
+    pdl_launch_dependents();
+    pdl_wait();
+    // the decode kernel has completed: its counter and (below) its scratch are put back for the next launch
+    if (clocked) { ws.ctrl->dec_ticket = 0; ws.ctrl->dec_time[5] = global_timer_ns(); }
+    const int4* pr = reinterpret_cast<const int4*>(ws.pair_row + (size_t)t * kTopK);
+    const float4* pw = reinterpret_cast<const float4*>(ws.pair_weight + (size_t)t * kTopK);
+    const int status = __ldcg(&ws.ctrl->status);
+    const int4 ra = __ldcg(pr), rb = __ldcg(pr + 1);
+    const float4 wa = __ldcg(pw), wb = __ldcg(pw + 1);
+    if (status != kStatusOk) return;   // the rows are not there (see decode_layer_kernel)
+    const int rows[kTopK] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+    const float wts[kTopK] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+    uint4 raw[kTopK];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
-            const int np = sh->pair_count[t];
-            for (int p = 0; p < np; ++p) {
-                const float w = sh->pair_w[t][p];
-                const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(ws.y + (size_t)sh->pair_row[t][p] * kHidden) + ch);
-                const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    for (int p = 0; p < kTopK; ++p)
+        if (rows[p] >= 0) raw[p] = __ldcg(reinterpret_cast<const uint4*>(ws.y + (size_t)rows[p] * kHidden) + ch);
+    if (ch < kInter / 4) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 f = __bfloat1622float2(h2[j]);
-                    acc[2 * j] += f.x * w;
-                    acc[2 * j + 1] += f.y * w;
-                }
+        for (int p = 0; p < kTopK; ++p)
+            if (rows[p] >= 0)
+                reinterpret_cast<uint4*>(ws.dec_act + (size_t)rows[p] * kInter)[ch] = make_uint4(kAbsent, kAbsent, kAbsent, kAbsent);
+    }
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+#pragma unroll
+    for (int p = 0; p < kTopK; ++p) {
+        if (rows[p] >= 0) {
+            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw[p]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(h2[j]);
+                acc[2 * j] += f.x * wts[p];
+                acc[2 * j + 1] += f.y * wts[p];
             }
-            uint4 packed;
-            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&packed);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-            reinterpret_cast<uint4*>(a.out + (size_t)t * kHidden)[ch] = packed;
         }
     }
-    stamp(6);
+    uint4 packed;
+    __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
+    reinterpret_cast<uint4*>(out + (size_t)t * kHidden)[ch] = packed;
+    if (clocked) ws.ctrl->dec_time[6] = global_timer_ns();
 }
 
 }  // namespace
@@ -670,12 +741,17 @@ cudaError_t launch_decode_layer(const DecodeArgs& args, const void* tmap_w1, con
     cfg.dynamicSmemBytes = sizeof(DecodeShared);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;   // all CTAs co-resident: the grid barriers need it
-    attr[0].val.cooperative = 1;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // set-up under the predecessor's tail
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, decode_layer_kernel, args, *static_cast<const CUtensorMap*>(tmap_w1),
-                              *static_cast<const CUtensorMap*>(tmap_w2), ws);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, decode_layer_kernel, args, *static_cast<const CUtensorMap*>(tmap_w1),
+                                             *static_cast<const CUtensorMap*>(tmap_w2), ws);
+    if (e != cudaSuccess) return e;
+    cfg.gridDim = dim3(kDecCombineParts, args.T);
+    cfg.blockDim = dim3(kDecCombineThreads);
+    cfg.dynamicSmemBytes = 0;
+    return cudaLaunchKernelEx(&cfg, decode_combine_kernel, ws, args.out);
 }
 
 }  // namespace moe

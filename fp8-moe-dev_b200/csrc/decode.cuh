@@ -10,6 +10,8 @@ namespace moe {
 
 constexpr int kDecodeMaxTokens = 8;   // every expert then has at most 8 rows: one n = 8 MMA tile
 
+constexpr size_t kDecodeActBytes = sizeof(float) * kDecodeMaxTokens * kTopK * kInter;   // Workspace::dec_act
+
 struct DecodeArgs {
     const float* logits;            // [T, 256]
     const __nv_bfloat16* bias;      // [256]

@@ -77,9 +77,8 @@ struct Control {
     int splitk_ticket[kSplitKSlots];     // per-tile arrival counters of the split-K reduction (self-clearing)
     int unit_ticket[2];                  // next work unit of the fused expert GEMMs (zeroed by the routing kernel's scan)
     int push_done;                       // combine-and-push CTAs finished (ticket, self-clearing)
-    unsigned dec_count;                  // arrival counters of the decode kernel's two grid barriers
-    unsigned dec_phase;                  // (cleared by CTA 0 of each launch, see decode.cu)
-    int pad2;
+    unsigned dec_ticket;                 // next run of work units of the decode kernel (cleared by its combine)
+    int pad2[2];
     unsigned long long dec_time[16];     // phase timestamps (ns) of CTA 0 in the last decode-kernel run
     // Timestamps (ns, %globaltimer) of the last fused combine + reduce-scatter on this rank:
     // [0] first CTA of the push starts, [1] last CTA of the push done (flags published), [2] first CTA of the
@@ -138,7 +137,7 @@ struct Workspace {
     uint32_t* pair_code;    // [T,8] (local expert << 24) | slot inside the expert
     float* pair_weight;     // [T,8] weight * (renorm) * routed_scaling_factor
     int* pair_row;          // [T,8] packed row of each kept pair, -1 past the token's pair count (written by the
-                            //       permute kernel; lets the fused exchange find a token's rows in one load)
+                            //       permute and decode kernels; lets a combine find a token's rows in one load)
     int* row_token;         // [M_cap] token of each packed row (diagnostics / tests)
     uint8_t* a1;            // [M_cap, H]   e4m3 rows gathered per expert
     float* sfa1;            // [56, M_cap]  their 1x128 scales, k-block major
@@ -146,6 +145,7 @@ struct Workspace {
     float* sfa2;            // [16, M_cap]
     __nv_bfloat16* y;       // [M_cap, H]   GEMM2 rows before the weighted combine
     float* splitk_partial;  // [kSplitKSlots, 4, 256] fp32 partial rows of split-K work units
+    float* dec_act;         // [64, 2048] fp32 SwiGLU output of the decode kernel, all bits set where nothing was stored yet
     int m_cap;              // packed-row capacity (multiple of 128)
     int max_tiles;
     Geometry geo;

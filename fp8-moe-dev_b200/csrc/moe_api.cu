@@ -66,7 +66,7 @@ struct Carve {
 
 struct Layout {
     size_t ctrl, expert_offset, tile_info, tile_done, num_tiles, expert_map, topk_idx, topk_weight, pair_count, pair_code,
-        pair_weight, pair_row, row_token, a1, sfa1, a2, sfa2, y, splitk, sw1_packed, sw2_packed, total;
+        pair_weight, pair_row, row_token, a1, sfa1, a2, sfa2, y, splitk, dec_act, sw1_packed, sw2_packed, total;
     int m_cap, max_tiles;
 };
 
@@ -98,6 +98,7 @@ Layout make_layout(int T, int E, const Geometry& geo = kReferenceGeometry)
     L.sfa2 = c.take(sizeof(float) * (inter / kBlock) * L.m_cap);
     L.y = c.take(sizeof(__nv_bfloat16) * (size_t)L.m_cap * hidden);
     L.splitk = c.take(sizeof(float) * (size_t)kSplitKSlots * 4 * 256);  // kSplitKMaxRows rows of 256 floats per unit
+    L.dec_act = c.take(kDecodeActBytes);
     L.sw1_packed = c.take(sizeof(float) * packed_scale_floats(1, E, geo));
     L.sw2_packed = c.take(sizeof(float) * packed_scale_floats(2, E, geo));
     L.total = c.off;
@@ -267,11 +268,12 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
     cudaError_t e = cudaSuccess;
     if (h->counters_dirty) {
         e = cudaMemsetAsync(h->ws.ctrl, 0, sizeof(Control), stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->ws.dec_act, 0xff, kDecodeActBytes, stream);
         h->counters_dirty = false;
     }
     if (h->opt_decode && h->decode_ctas_per_sm > 0 && T <= kDecodeMaxTokens && finalize && !ex && placement == 1 &&
         h->opt_stop_after == 0 && ref_geo && h->reference_routing()) {
-        // the whole layer as one cooperative kernel, one CTA per SM
+        // the whole layer but the combine as one persistent kernel, one CTA per SM
         DecodeArgs d;
         d.logits = a.routing_logits;
         d.bias = static_cast<const __nv_bfloat16*>(a.routing_bias);
@@ -290,20 +292,12 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
         d.pol = pol;
         mark(0);
         if (e == cudaSuccess) e = launch_decode_layer(d, h->tmap_dec_w1, h->tmap_dec_w2, h->ws, h->num_sms, stream);
-        if (e == cudaErrorCooperativeLaunchTooLarge) {
-            // fewer SMs than the device reports are available to this context (partitioned GPU):
-            // the grid cannot be co-resident, so this handle uses the chain from now on
-            cudaGetLastError();
-            h->decode_ctas_per_sm = 0;
-            e = cudaSuccess;
-        } else {
-            for (int i = 1; i <= 6; ++i) mark(i);
-            if (e != cudaSuccess) {
-                h->counters_dirty = true;
-                return fail(h, MOE_FP8_B200_ERR_CUDA, "decode launch failed: %s", cudaGetErrorString(e));
-            }
-            return MOE_FP8_B200_OK;
+        for (int i = 1; i <= 6; ++i) mark(i);
+        if (e != cudaSuccess) {
+            h->counters_dirty = true;
+            return fail(h, MOE_FP8_B200_ERR_CUDA, "decode launch failed: %s", cudaGetErrorString(e));
         }
+        return MOE_FP8_B200_OK;
     }
     if (e == cudaSuccess && (a.gemm1_weights_scale != h->cached_s1 || a.gemm2_weights_scale != h->cached_s2)) {
         // new scale tensors: lay them out for the GEMMs' promotion (stream-ordered in front of the chain)
@@ -531,6 +525,7 @@ int moe_fp8_b200_create_shaped(moe_fp8_b200_handle* out, int device, int max_tok
     w.sfa2 = reinterpret_cast<float*>(h->base + L.sfa2);
     w.y = reinterpret_cast<__nv_bfloat16*>(h->base + L.y);
     w.splitk_partial = reinterpret_cast<float*>(h->base + L.splitk);
+    w.dec_act = reinterpret_cast<float*>(h->base + L.dec_act);
     w.expert_map = reinterpret_cast<int*>(h->base + L.expert_map);
     h->sw1_packed = reinterpret_cast<float*>(h->base + L.sw1_packed);
     h->sw2_packed = reinterpret_cast<float*>(h->base + L.sw2_packed);
@@ -539,6 +534,7 @@ int moe_fp8_b200_create_shaped(moe_fp8_b200_handle* out, int device, int max_tok
     w.geo = h->geo;
     // Small control arrays start defined; the large row buffers are written before use.
     e = cudaMemset(h->base, 0, L.topk_idx);
+    if (e == cudaSuccess) e = cudaMemset(w.dec_act, 0xff, kDecodeActBytes);
     if (e == cudaSuccess) e = cudaMemset(w.row_token, 0xff, sizeof(int) * (size_t)L.m_cap);
     if (e == cudaSuccess) e = configure_gemm_kernels();
     if (e == cudaSuccess) e = configure_expert_gemms();
@@ -1044,7 +1040,7 @@ int moe_fp8_b200_inject_device_status(moe_fp8_b200_handle h, int status, unsigne
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaMemcpyAsync(&h->ws.ctrl->status, &status, sizeof(int), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&h->ws.ctrl->dec_count, &stale_barrier_arrivals, sizeof(unsigned), cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync(&h->ws.ctrl->dec_ticket, &stale_barrier_arrivals, sizeof(unsigned), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "status injection: %s", cudaGetErrorString(e));
     return MOE_FP8_B200_OK;

@@ -200,6 +200,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- misc
+// Brings the 128-byte line of `p` into L2 (no value is returned, nothing is ordered by it).
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // 32-byte global store (sm_100): an epilogue thread owns a contiguous piece of one output row, and
 // the memory pipeline handles a warp's store row by row, so twice the bytes per instruction halve
 // the time the stores occupy it.  `p` must be 32-byte aligned.

@@ -103,7 +103,7 @@ class MoeLayer:
             self._raise(rc)
 
     def set_decode_kernel(self, on: bool):
-        """Batches of at most 8 tokens: one cooperative kernel (default) or the staged chain."""
+        """Batches of at most 8 tokens: one persistent kernel (default) or the staged chain."""
         rc = self._lib.moe_fp8_b200_set_option(self._h, _lib.OPT_DECODE_KERNEL, int(bool(on)))
         if rc != _lib.OK:
             self._raise(rc)

@@ -78,8 +78,8 @@ enum {
      * 0 (default) runs the whole layer. */
     MOE_FP8_B200_OPT_STOP_AFTER_STAGE = 4,
     /* 1 (default): batches of at most MOE_FP8_B200_DECODE_MAX_TOKENS tokens run as one
-     * cooperative kernel (routing, both GEMMs on warp-level MMAs straight from global memory,
-     * combine; two bounded grid barriers) instead of the five-kernel chain.  Same results up
+     * persistent kernel (routing, both GEMMs on warp-level MMAs; bounded waits) and a small
+     * combine kernel instead of the staged chain.  Same results up
      * to fp32 summation order inside GEMM1.  That kernel fills only the routing and pair
      * tables of the workspace (EXPERT_COUNT, TOPK_*, PAIR_*); 0 selects the chain, which also
      * leaves the packed rows, tiles and offsets behind for moe_fp8_b200_read_intermediate.
