@@ -49,7 +49,6 @@ constexpr int kHalfWarps = 8;                           // the CTA works as two 
 constexpr int kHalfThreads = kHalfWarps * 32;
 constexpr int kDecMaxActive = kDecodeMaxTokens * kTopK; // 64 (token, expert) pairs at most
 constexpr int kHidStride = kHidden + 64;                // row strides that spread rows over the banks
-constexpr int kA2Stride = kInter + 64;
 constexpr int kG1Cols = 8;                              // SwiGLU columns of a phase-1 unit
 constexpr int kG1Units = kInter / kG1Cols;              // 256 per expert
 constexpr int kG2Cols = 16;                             // output columns of a phase-2 unit
@@ -67,16 +66,12 @@ constexpr int kFewTokens = 4;
 constexpr int kCoopRouteTokens = 3;                     // up to here the CTA's warps route the tokens together
 static_assert(kHidden % kStepK == 0 && kInter % kStepK == 0, "K splits into whole steps");
 
-// Shared-memory pool: the hidden rows of all tokens (phase 2: each half's requantised rows of its expert), then
-// the two weight rings.
+// Shared-memory pool: the hidden rows of all tokens, then the two weight rings.
 __host__ __device__ constexpr int rows_tokens(int T) { return T <= kFewTokens ? kFewTokens : kDecodeMaxTokens; }
 constexpr int kPoolFew = kFewTokens * kHidStride + 2 * kRingFew * kStepBytes;
 constexpr int kPoolAll = kDecodeMaxTokens * kHidStride + 2 * kRing * kStepBytes;
 constexpr int kPoolBytes = kPoolFew > kPoolAll ? kPoolFew : kPoolAll;
 static_assert(kDecodeMaxTokens * kHidStride % 128 == 0 && kFewTokens * kHidStride % 128 == 0, "ring slots are 128-byte aligned");
-// half 1's rows lie rows_tokens(T) rows behind half 0's; the MMAs read eight rows from either start
-static_assert((kFewTokens + 8) * kA2Stride <= kFewTokens * kHidStride && 16 * kA2Stride <= kDecodeMaxTokens * kHidStride,
-              "phase 2 rows reuse the hidden-row area");
 static_assert(2 * kDecodeMaxTokens * kNumExperts * 4 <= 2 * kRing * kStepBytes, "routing scratch fits the idle rings");
 
 struct DecodeShared {
@@ -95,7 +90,6 @@ struct DecodeShared {
     int r_idx[kDecodeMaxTokens][kTopK];
     float r_sel[kDecodeMaxTokens][kTopK];
     float hid_scale[kDecodeMaxTokens][kHiddenBlocks];      // [token][kb]
-    float a2_scale[2][kDecodeMaxTokens][kInterBlocks];     // per half: [slot][kb] of the requantised rows
     alignas(16) int4 step_desc[2][kRingFew];               // {unit, step, next unit or -1, -}; unit -1: no more
     alignas(8) uint64_t full_bar[2][kRingFew];
     alignas(8) uint64_t empty_bar[2][kRingFew];
@@ -148,20 +142,19 @@ __device__ __forceinline__ void mma_e4m3(float (&c)[4], uint32_t a0, uint32_t a1
 // and a dot product does not care about more.  (The choice cannot depend on the row: a product
 // pairs the A bytes of one lane group with the B bytes of another.  The weight rows are 1 KB apart,
 // so rows r and r + 1, which share a shared-memory access phase, collide two-way; that is cheap.)
+__device__ __forceinline__ void mma_half(float (&acc)[4], const uint8_t* arow, const uint4& b) {
+    const uint4 lo = *reinterpret_cast<const uint4*>(arow);
+    const uint4 hi = *reinterpret_cast<const uint4*>(arow + 8 * kStepStride);
+    mma_e4m3(acc, lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+    mma_e4m3(acc, lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+}
 __device__ __forceinline__ void mma_block(float (&acc)[4], const uint8_t* arow, const uint8_t* brow) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int off = 64 * h;
-        const uint4 lo = *reinterpret_cast<const uint4*>(arow + off);
-        const uint4 hi = *reinterpret_cast<const uint4*>(arow + 8 * kStepStride + off);
-        const uint4 b = *reinterpret_cast<const uint4*>(brow + off);
-        mma_e4m3(acc, lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-        mma_e4m3(acc, lo.z, hi.z, lo.w, hi.w, b.z, b.w);
-    }
+    mma_half(acc, arow, *reinterpret_cast<const uint4*>(brow));
+    mma_half(acc, arow + 64, *reinterpret_cast<const uint4*>(brow + 64));
 }
 
 // How the work is drawn.  Workers (half CTAs) draw tickets from a counter; a ticket stands for a run of
-// consecutive units.  Of each phase the first tickets, one per worker, stand for long runs (three quarters of
+// consecutive units.  Of each phase the first tickets, one per worker, stand for long runs (seven eighths of
 // the phase: few changes of expert, whose rows phase 2 has to requantise again), the rest for short ones that
 // even out how fast the workers get their weights.  All of phase 1 is drawn before phase 2, and phase 2 waits
 // only for phase-1 units, i.e. for workers that are running: the waits end whatever part of the grid is
@@ -171,10 +164,10 @@ struct PhasePlan {
     int units, in_runs, runs, rest_run, tickets;
     __device__ __forceinline__ void make(int n, int workers) {
         units = n;
-        in_runs = n >= 2 * workers ? n / 4 * 3 : 0;
+        in_runs = n >= 2 * workers ? n / 8 * 7 : 0;
         runs = in_runs > 0 ? workers : 0;
         const int rest = n - in_runs;
-        rest_run = rest / (workers * 6);
+        rest_run = rest / (workers * 4);
         if (rest_run < 1) rest_run = 1;
         tickets = runs + (rest + rest_run - 1) / rest_run;
     }
@@ -227,6 +220,9 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
         for (int t = 0; t < T; ++t) prefetch_l2(a.hidden + (size_t)t * kHidden + (size_t)(tid - 192) * 128);
     }
     pdl_wait();
+    // the first ticket travels while the tables are made (an unused one does no harm)
+    int first_ticket = 0;
+    if (warp >= kDecWarps && lane == 0) first_ticket = (int)atomicAdd(&ws.ctrl->dec_ticket, 1u);
     // A failure that an earlier launch recorded stays in the status word until the host has read it
     // (moe_fp8_b200_check clears it together with any arrival counts that launch left on the grid
     // barriers).  Until then this kernel does nothing: with stale counts its barriers would open early.
@@ -446,7 +442,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
             if (ticket < p1.tickets) { p1.range(ticket, begin, end); bit = 0; }
             else { p2.range(ticket - p1.tickets, begin, end); bit = kPhase2Bit; }
         };
-        int ticket = n_active > 0 ? (int)atomicAdd(&ws.ctrl->dec_ticket, 1u) : tickets;
+        int ticket = first_ticket;
         while (ok && ticket < tickets) {
             int u, end, bit;
             range_of(ticket, u, end, bit);
@@ -507,6 +503,15 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
         if (lane == 0) mbar_arrive(smem_u32(&empty_bar[slot]));
         if (++slot == ring) { slot = 0; phase ^= 1u; }
     };
+    // waits for the next step; false: this half gives up
+    auto arrived = [&]() -> bool { return mbar_wait(smem_u32(&full_bar[slot]), phase, abort_flag); };
+    // the first step of the next unit and what the producer wrote about it ({-1, ...} once there is no more work)
+    int4 d = make_int4(-1, 0, -1, 0);
+    auto next_unit = [&]() {
+        ok = ok && arrived();
+        d.x = -1;
+        if (ok) d = sh->step_desc[half][slot];
+    };
     // The weight scales of a unit's K blocks sit in lanes of the warp that uses them (phase 1: lanes 0..13, 7
     // linear and 7 gated; phase 2: lanes 0 and 1), fetched one unit ahead so that no step waits for them.
     auto unit_scales = [&](int unit) -> float {
@@ -528,129 +533,150 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
     // the hidden rows must have landed before the first MMA
     if (!mbar_wait(smem_u32(&sh->hid_bar), 0u, abort_flag)) ok = false;
 
-    uint8_t* a2rows = sh->pool + half * (rows_tokens(T) * kA2Stride);
-    float(*a2s)[kInterBlocks] = sh->a2_scale[half];
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    float sc_cur = 0.0f, sc_next = 0.0f;
-    int ai = 0, in = 0, m = 0, staged = -1, parity = 0;
+    float sc_next = 0.0f;
     int loaded_for = -1;   // unit that sc_next belongs to
-    bool in_phase2 = false;
-    while (ok) {
-        if (!mbar_wait(smem_u32(&full_bar[slot]), phase, abort_flag)) { ok = false; break; }
-        const int4 d = sh->step_desc[half][slot];
-        if (d.x < 0) break;
-        const uint8_t* wst = wring + slot * kStepBytes;
-        const int i = d.y;
-        const bool p2 = (d.x & kPhase2Bit) != 0;
-        if (i == 0) {   // a new unit
-            const int u = p2 ? d.x - kPhase2Bit : d.x;
-            ai = p2 ? u / kG2Units : u / kG1Units;
-            in = p2 ? u - ai * kG2Units : u - ai * kG1Units;
-            m = sh->act_m[ai];
-            sc_cur = loaded_for == d.x ? sc_next : unit_scales(d.x);
-            acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
-            if (p2 && ai != staged) {
-                // ---------------------------------------------------- another expert's rows for phase 2
-                if (!in_phase2) {
-                    // the hidden rows are overwritten below: both halves have to be through with them
-                    stamp(2);
-                    named_bar_sync(3, kConsumers);
-                    in_phase2 = true;
-                }
-                named_bar_sync(bar_id, kHalfThreads);   // the half is done with the previous expert's rows
-                if (staged < 0) stamp(3);
-                // 1x128 requantisation of the expert's rows, as in the staged GEMM1 epilogue:
-                // scale = amax / 448 (1 if the block is zero), payload e4m3(v * (1 / scale))
-                for (int item = hw; item < m * kInterBlocks; item += kHalfWarps) {
-                    const int row = item / kInterBlocks, ib = item % kInterBlocks;
-                    const float* src = act + (size_t)(sh->act_row0[ai] + row) * kInter + ib * kBlock + lane * 4;
-                    float4 v = ld_relaxed_gpu(src);
-                    if (!__all_sync(0xffffffffu, is_there(v))) {   // phase-1 units of other workers still under way
-                        const uint64_t t0 = global_timer_ns();
-                        do {
-                            if (!is_there(v)) v = ld_relaxed_gpu(src);
-                            if (*abort_flag != 0 || global_timer_ns() - t0 > kWaitLimitNs) sh->abort = 1;
-                        } while (!__all_sync(0xffffffffu, is_there(v) || *abort_flag != 0));
-                    }
-                    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+    int parity = 0;
+    // ------------------------------------------------------------------ phase 1: GEMM1 + SwiGLU
+    for (next_unit(); d.x >= 0 && !(d.x & kPhase2Bit); next_unit()) {
+        const int ai = d.x / kG1Units, g = d.x % kG1Units, m = sh->act_m[ai];
+        const float sc_cur = loaded_for == d.x ? sc_next : unit_scales(d.x);
+        const uint8_t* brow = sh->pool + sh->act_tok[ai][r < m ? r : 0] * kHidStride + hw * kBlock + 16 * c;
+        const float* sc0 = sh->hid_scale[sh->act_tok[ai][2 * c < m ? 2 * c : 0]] + hw;
+        const float* sc1 = sh->hid_scale[sh->act_tok[ai][2 * c + 1 < m ? 2 * c + 1 : 0]] + hw;
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        int next = -1;
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                    const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
-                    const float inv = 1.0f / sc;
-                    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v.x * inv, v.y * inv), __NV_SATFINITE, __NV_E4M3);
-                    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v.z * inv, v.w * inv), __NV_SATFINITE, __NV_E4M3);
-                    *reinterpret_cast<uint32_t*>(a2rows + row * kA2Stride + ib * kBlock + lane * 4) = lo | (hi << 16);
-                    if (lane == 0) a2s[row][ib] = sc;
-                }
-                named_bar_sync(bar_id, kHalfThreads);
-                if (*abort_flag != 0) { ok = false; break; }
-                staged = ai;
-            }
-        }
-        const int kb = hw + kHalfWarps * i;
-        float raw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (!p2) {
-            // -------------------------------------------------------- phase 1: GEMM1 + SwiGLU
-            const float sl = __shfl_sync(0xffffffffu, sc_cur, i), sg = __shfl_sync(0xffffffffu, sc_cur, kG1Steps + i);
-            const int tok = sh->act_tok[ai][r < m ? r : 0];
-            mma_block(raw, wst + r * kStepStride + hw * kBlock + 16 * c, sh->pool + tok * kHidStride + kb * kBlock + 16 * c);
+        for (int i = 0; i < kG1Steps; ++i) {
+            if (i > 0 && !arrived()) { ok = false; break; }
+            float raw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            mma_block(raw, wring + slot * kStepBytes + r * kStepStride + hw * kBlock + 16 * c, brow + i * kHalfWarps * kBlock);
+            if (i == kG1Steps - 1) next = sh->step_desc[half][slot].z;
             release();
-            const int t0 = sh->act_tok[ai][2 * c < m ? 2 * c : 0], t1 = sh->act_tok[ai][2 * c + 1 < m ? 2 * c + 1 : 0];
-            const float sa0 = sh->hid_scale[t0][kb], sa1 = sh->hid_scale[t1][kb];
+            const float sl = __shfl_sync(0xffffffffu, sc_cur, i), sg = __shfl_sync(0xffffffffu, sc_cur, kG1Steps + i);
+            const float sa0 = sc0[i * kHalfWarps], sa1 = sc1[i * kHalfWarps];
             acc[0] = fmaf(raw[0], sa0 * sl, acc[0]);
             acc[1] = fmaf(raw[1], sa1 * sl, acc[1]);
             acc[2] = fmaf(raw[2], sa0 * sg, acc[2]);
             acc[3] = fmaf(raw[3], sa1 * sg, acc[3]);
-        } else {
-            // -------------------------------------------------------- phase 2: GEMM2
-            const float sw = __shfl_sync(0xffffffffu, sc_cur, i);
-            mma_block(raw, wst + r * kStepStride + hw * kBlock + 16 * c, a2rows + r * kA2Stride + kb * kBlock + 16 * c);
+        }
+        if (!ok) break;
+        if (next >= 0) { sc_next = unit_scales(next); loaded_for = next; }
+        // the unit is complete: add the eight warps' partial sums
+        float* red = &sh->red[half][parity][0][0];
+        parity ^= 1;
+        *reinterpret_cast<float4*>(red + hw * 128 + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        named_bar_sync(bar_id, kHalfThreads);
+        if (htid < 64) {
+            const int l = htid & 31, jj = htid >> 5;
+            float lin = 0.0f, gate = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kHalfWarps; ++w) {
+                lin += red[w * 128 + l * 4 + jj];
+                gate += red[w * 128 + l * 4 + 2 + jj];
+            }
+            const int row = 2 * (l & 3) + jj, col = g * kG1Cols + (l >> 2);
+            if (row < m) {
+                const float x1 = round_bf16(lin), x2 = round_bf16(gate);
+                const float silu = a.silu_exact ? x2 / (1.0f + __expf(-x2))
+                                                : x2 * (0.5f * (x2 * rsqrtf(fmaf(x2, x2, 4.0f)) + 1.0f));
+                st_relaxed_gpu(act + (size_t)(sh->act_row0[ai] + row) * kInter + col, silu * x1);
+            }
+        }
+    }
+
+    // ------------------------------------------------------------------ phase 2: requantisation + GEMM2
+    stamp(2);
+    int staged = -1;
+    uint4 bfrag[kG2Steps][2];      // this warp's K blocks of the staged expert's rows
+    float bscale[kG2Steps][2];     // ... and the scales of rows 2c and 2c + 1
+    for (; ok && d.x >= 0; next_unit()) {
+        const int u = d.x - kPhase2Bit, ai = u / kG2Units, hg = u % kG2Units, m = sh->act_m[ai];
+        if (ai != staged) {
+            // 1x128 requantisation as in the staged GEMM1 epilogue: scale = amax / 448 (1 if the block is
+            // zero), payload e4m3(v * (1 / scale)).  A warp needs its own two K blocks only and keeps them
+            // in registers as B fragments, so the warps take another expert up without meeting.
+#pragma unroll
+            for (int k2 = 0; k2 < kG2Steps; ++k2) {
+                const float* src = act + (size_t)sh->act_row0[ai] * kInter + (hw + kHalfWarps * k2) * kBlock + lane * 4;
+                bfrag[k2][0] = bfrag[k2][1] = make_uint4(0u, 0u, 0u, 0u);
+                bscale[k2][0] = bscale[k2][1] = 0.0f;
+#pragma unroll
+                for (int j0 = 0; j0 < kDecodeMaxTokens; j0 += 4) {
+                    if (j0 >= m) break;
+                    float4 v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (j0 + j < m) v[j] = ld_relaxed_gpu(src + (size_t)(j0 + j) * kInter);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (j0 + j >= m) break;
+                        if (!__all_sync(0xffffffffu, is_there(v[j]))) {   // phase-1 units still under way elsewhere
+                            const uint64_t t0 = global_timer_ns();
+                            do {
+                                if (!is_there(v[j])) v[j] = ld_relaxed_gpu(src + (size_t)(j0 + j) * kInter);
+                                if (*abort_flag != 0 || global_timer_ns() - t0 > kWaitLimitNs) sh->abort = 1;
+                            } while (!__all_sync(0xffffffffu, is_there(v[j]) || *abort_flag != 0));
+                        }
+                        float amax = fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w)));
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                        const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
+                        const float inv = 1.0f / sc;
+                        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[j].x * inv, v[j].y * inv), __NV_SATFINITE, __NV_E4M3);
+                        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[j].z * inv, v[j].w * inv), __NV_SATFINITE, __NV_E4M3);
+                        const uint32_t w = lo | (hi << 16);   // bytes 4 lane .. 4 lane + 3 of the row's block
+                        // lanes of fragment row j0 + j take bytes 16c .. 16c+15 and 64+16c .. 64+16c+15
+                        uint32_t g[8];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) g[q] = __shfl_sync(0xffffffffu, w, (q >> 2) * 16 + 4 * c + (q & 3));
+                        if (r == j0 + j) {
+                            bfrag[k2][0] = make_uint4(g[0], g[1], g[2], g[3]);
+                            bfrag[k2][1] = make_uint4(g[4], g[5], g[6], g[7]);
+                        }
+                        if (2 * c == j0 + j) bscale[k2][0] = sc;
+                        if (2 * c + 1 == j0 + j) bscale[k2][1] = sc;
+                    }
+                }
+            }
+            if (staged < 0) stamp(3);
+            staged = ai;
+        }
+        const float sc_cur = loaded_for == d.x ? sc_next : unit_scales(d.x);
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        int next = -1;
+#pragma unroll
+        for (int i = 0; i < kG2Steps; ++i) {
+            if (i > 0 && !arrived()) { ok = false; break; }
+            float raw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const uint8_t* arow = wring + slot * kStepBytes + r * kStepStride + hw * kBlock + 16 * c;
+            mma_half(raw, arow, bfrag[i][0]);
+            mma_half(raw, arow + 64, bfrag[i][1]);
+            if (i == kG2Steps - 1) next = sh->step_desc[half][slot].z;
             release();
-            const float sa0 = a2s[2 * c][kb] * sw, sa1 = a2s[2 * c + 1][kb] * sw;
+            const float sw = __shfl_sync(0xffffffffu, sc_cur, i);
+            const float sa0 = bscale[i][0] * sw, sa1 = bscale[i][1] * sw;
             acc[0] = fmaf(raw[0], sa0, acc[0]);
             acc[1] = fmaf(raw[1], sa1, acc[1]);
             acc[2] = fmaf(raw[2], sa0, acc[2]);
             acc[3] = fmaf(raw[3], sa1, acc[3]);
         }
-        const bool last = i == (p2 ? kG2Steps : kG1Steps) - 1;
-        if (d.z >= 0 && d.z != loaded_for) { sc_next = unit_scales(d.z); loaded_for = d.z; }
-        if (last) {   // the unit is complete: add the eight warps' partial sums
-            float* red = &sh->red[half][parity][0][0];
-            parity ^= 1;
-            *reinterpret_cast<float4*>(red + hw * 128 + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-            named_bar_sync(bar_id, kHalfThreads);
-            if (!p2) {
-                if (htid < 64) {
-                    const int l = htid & 31, jj = htid >> 5;
-                    float lin = 0.0f, gate = 0.0f;
+        if (!ok) break;
+        if (next >= 0) { sc_next = unit_scales(next); loaded_for = next; }
+        float* red = &sh->red[half][parity][0][0];
+        parity ^= 1;
+        *reinterpret_cast<float4*>(red + hw * 128 + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        named_bar_sync(bar_id, kHalfThreads);
+        if (htid < 128) {
+            const int l = htid >> 2, q = htid & 3;
+            const int row = 2 * (l & 3) + (q & 1), hrow = hg * kG2Cols + (l >> 2) + 8 * (q >> 1);
+            float sum = 0.0f;
 #pragma unroll
-                    for (int w = 0; w < kHalfWarps; ++w) {
-                        lin += red[w * 128 + l * 4 + jj];
-                        gate += red[w * 128 + l * 4 + 2 + jj];
-                    }
-                    const int row = 2 * (l & 3) + jj, col = in * kG1Cols + (l >> 2);
-                    if (row < m) {
-                        const float x1 = round_bf16(lin), x2 = round_bf16(gate);
-                        const float silu = a.silu_exact ? x2 / (1.0f + __expf(-x2))
-                                                        : x2 * (0.5f * (x2 * rsqrtf(fmaf(x2, x2, 4.0f)) + 1.0f));
-                        st_relaxed_gpu(act + (size_t)(sh->act_row0[ai] + row) * kInter + col, silu * x1);
-                    }
-                }
-            } else if (htid < 128) {
-                const int l = htid >> 2, q = htid & 3;
-                const int row = 2 * (l & 3) + (q & 1), hrow = in * kG2Cols + (l >> 2) + 8 * (q >> 1);
-                float sum = 0.0f;
-#pragma unroll
-                for (int w = 0; w < kHalfWarps; ++w) sum += red[w * 128 + l * 4 + q];
-                if (row < m) ws.y[(size_t)(sh->act_row0[ai] + row) * kHidden + hrow] = __float2bfloat16_rn(sum);
-            }
+            for (int w = 0; w < kHalfWarps; ++w) sum += red[w * 128 + l * 4 + q];
+            if (row < m) ws.y[(size_t)(sh->act_row0[ai] + row) * kHidden + hrow] = __float2bfloat16_rn(sum);
         }
     }
-    if (!in_phase2) {   // the other half may be waiting to overwrite the hidden rows
-        stamp(2);
-        named_bar_sync(3, kConsumers);
-        stamp(3);
-    }
+    if (staged < 0) stamp(3);   // no phase-2 unit came this way
+    if (*abort_flag != 0) ok = false;
     if (!ok) {
         // a half that gave up on a wait says so; the producers let their copies land before they leave
         atomicCAS(&ws.ctrl->status, kStatusOk, kStatusDecodeTimeout);
