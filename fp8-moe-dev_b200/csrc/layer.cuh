@@ -72,7 +72,7 @@ struct Control {
     int status;                          // 0 ok; otherwise the first error a kernel recorded
     int status_detail;
     int blocks_done;                     // routing CTAs finished (ticket for the last-CTA scan)
-    int pad;
+    int permute_done;                    // permute CTAs finished, where zero_rows_kernel asks (zeroed by the routing kernel's scan)
     int expert_rows[kMaxLocalExperts];   // copy of the counters of the last call (diagnostics)
     int splitk_ticket[kSplitKSlots];     // per-tile arrival counters of the split-K reduction (self-clearing)
     int unit_ticket[2];                  // next work unit of the fused expert GEMMs (zeroed by the routing kernel's scan)
@@ -150,6 +150,19 @@ struct Workspace {
     int max_tiles;
     Geometry geo;
     int w_tiled;            // the GEMMs' weight map covers the tile-ordered copy (one 32 KB piece per tile and K block)
+};
+
+// Pieces of pinned host memory that fetch_inputs_kernel brings to the device (32-bit words; destinations 16-byte
+// aligned).
+struct FetchList {
+    static constexpr int kMax = 3;
+    struct { const uint32_t* src; uint32_t* dst; size_t words; } seg[kMax];
+    int n;
+    void add(const void* src, void* dst, size_t bytes) {
+        seg[n].src = static_cast<const uint32_t*>(src);
+        seg[n].dst = static_cast<uint32_t*>(dst);
+        seg[n++].words = bytes / 4;
+    }
 };
 
 // Tensor maps of one pair of GEMM launches (host addresses of CUtensorMap objects): packed activations and

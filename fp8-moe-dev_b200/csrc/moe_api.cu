@@ -1,6 +1,7 @@
 // C ABI of the layer (declared in include/moe_fp8_b200.h): handle + workspace, argument
 // validation, the reference's T-keyed dispatch policy resolved on the host, and the
 // stage chain enqueued on the caller's stream.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdarg>
@@ -16,8 +17,10 @@
 namespace moe {
 cudaError_t launch_route_dispatch(const float*, const void*, const Workspace&, int, int, int, float,
                                   const DispatchPolicy&, int, cudaStream_t);
-cudaError_t launch_permute(const void*, const float*, const Workspace&, int, cudaStream_t);
-cudaError_t launch_combine(const Workspace&, void*, int, cudaStream_t);
+cudaError_t launch_permute(const void*, const float*, const Workspace&, int, int, cudaStream_t);
+cudaError_t launch_combine(const Workspace&, void*, int, int, cudaStream_t);
+cudaError_t launch_zero_rows(const Workspace&, void*, int, cudaStream_t);
+cudaError_t launch_fetch_inputs(const FetchList&, int, cudaStream_t);
 cudaError_t launch_quantize_rows(const void*, void*, float*, int, int, cudaStream_t);
 cudaError_t launch_combine_push(const Workspace&, const ExchangeView&, int, cudaStream_t);
 cudaError_t launch_reduce_owned(const Workspace&, const ExchangeView&, int, void*, cudaStream_t);
@@ -41,6 +44,13 @@ using namespace moe;
 namespace {
 
 constexpr int kVersion = (0 << 16) | 1;
+
+// run_host with pinned buffers, rows without a local expert written beside the GEMMs: pays where a GPU holds at most
+// a quarter of the experts (half to a quarter of the tokens have no row; with 128 experts 3 %, no difference) and
+// the batch has enough such rows (32 experts, written aside / by the combine: T=57 185 / 182 us, T=256 264 / 302,
+// T=2048 789 / 1009; 64 experts: T=128 378 / 372, T=256 460 / 468, T=2048 1300 / 1384).
+constexpr int kZeroAsideExperts = 64;
+constexpr int kZeroAsideTokens = 256;
 thread_local std::string g_create_error;
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -163,6 +173,9 @@ struct moe_fp8_b200_ctx {
     // staging for run_host (allocated on its first use)
     uint8_t* stage = nullptr;
     size_t stage_bytes = 0;
+    // run_host with pinned buffers: the rows without a local expert are written on a stream of their own
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_begin = nullptr, side_done = nullptr;
     // pipelined host path: two staging sets, copy streams, per-set events
     uint8_t* pipe_stage[2] = {nullptr, nullptr};
     size_t pipe_bytes = 0;
@@ -212,8 +225,10 @@ void resolve_reference_policy(int T, DispatchPolicy& p)
     p.renorm = (T == 14107) ? 0 : 1;
 }
 
+// `zero_aside` (staged chain only, handle's side stream present): the output rows of tokens without a local expert
+// are written on the side stream while the GEMMs run, the combine leaves them out, and `stream` waits for both.
 int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_t stream,
-                  const ExchangeView* ex = nullptr, bool finalize = true)
+                  const ExchangeView* ex = nullptr, bool finalize = true, bool zero_aside = false)
 {
     const int T = a.num_tokens;
     const int E = h->num_local_experts;
@@ -321,6 +336,12 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
         e = launch_route_dispatch(a.routing_logits, a.routing_bias, h->ws, T, (int)a.local_expert_offset, E,
                                   (float)a.routed_scaling_factor, pol, /*do_scan=*/1, stream);
     mark(1);
+    if (zero_aside) {
+        if (e == cudaSuccess) e = cudaEventRecord(h->side_begin, stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->side_begin, 0);
+        if (e == cudaSuccess) e = launch_zero_rows(h->ws, a.output, T, h->side);
+        if (e == cudaSuccess) e = cudaEventRecord(h->side_done, h->side);
+    }
     mark(2);
     const int stop = h->opt_stop_after > 0 ? h->opt_stop_after : 99;
     // decode-sized batches may leave most SMs without a tile: there the split-K instantiation
@@ -328,13 +349,15 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
     const int split_k = (T <= 4 && ref_geo) ? 1 : 0;   // 4 = kSplitKMaxRows of the GEMM kernel
     // at most 64 tokens (an expert then has at most 64 rows): 64-row activation boxes and a fourth operand stage
     const int small_a = (h->opt_small_batch_ring && T > 4 && T <= 64 && ref_geo) ? 1 : 0;
-    if (e == cudaSuccess && stop >= 2) e = launch_permute(a.hidden_states, a.hidden_states_scale, h->ws, T, stream);
+    if (e == cudaSuccess && stop >= 2) e = launch_permute(a.hidden_states, a.hidden_states_scale, h->ws, T, zero_aside ? 1 : 0, stream);
     mark(3);
     const GemmMaps maps = {small_a ? h->tmap_a1_small : h->tmap_a1, tiled ? h->tmap_w1_tiled : h->tmap_w1,
                            small_a ? h->tmap_a2_small : h->tmap_a2, tiled ? h->tmap_w2_tiled : h->tmap_w2, h->tmap_y};
-    // one persistent CTA per SM; CTAs without work leave at once
+    // one persistent CTA per SM (a CTA takes all of an SM's registers: one SM is left to zero_rows_kernel where that
+    // runs); CTAs without work leave at once
+    const int gemm_ctas = zero_aside && h->num_sms > 1 ? h->num_sms - 1 : h->num_sms;
     auto gemms = [&](int phases) {
-        return launch_expert_gemms(maps, gemm_ws, h->sw1_packed, h->sw2_packed, h->opt_exact_silu, phases, h->num_sms, small_a, stream);
+        return launch_expert_gemms(maps, gemm_ws, h->sw1_packed, h->sw2_packed, h->opt_exact_silu, phases, gemm_ctas, small_a, stream);
     };
     if (split_k) {
         if (e == cudaSuccess && stop >= 3)
@@ -355,15 +378,48 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
             e = launch_combine_push(h->ws, *ex, T, stream);
             if (e == cudaSuccess) e = launch_reduce_owned(h->ws, *ex, T, a.output, stream);
         } else {
-            e = launch_combine(h->ws, a.output, T, stream);
+            e = launch_combine(h->ws, a.output, T, zero_aside ? 1 : 0, stream);
         }
     }
+    if (e == cudaSuccess && zero_aside) e = cudaStreamWaitEvent(stream, h->side_done, 0);
     mark(6);
     if (e != cudaSuccess) {
         h->counters_dirty = true;
         return fail(h, MOE_FP8_B200_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
     }
     return MOE_FP8_B200_OK;
+}
+
+// The device's address of host memory that kernels can reach: [p, p + bytes) lies inside one pinned, mapped
+// allocation.  Anything else (pageable, managed, device memory, a range that leaves its allocation) is not taken.
+bool pinned_range(const void* p, size_t bytes, const void*& dev)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer) return false;
+    typedef CUresult (*AttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
+    static const AttributeFn get = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const cudaError_t e = cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &q);
+        return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<AttributeFn>(fn) : nullptr;
+    }();
+    if (!get) return false;
+    const CUdeviceptr d = reinterpret_cast<CUdeviceptr>(at.devicePointer);
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
+        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS)
+        return false;
+    if (d < start || bytes > size || d - start > size - bytes) return false;
+    dev = at.devicePointer;
+    return true;
+}
+
+bool overlap(const void* a, size_t na, const void* b, size_t nb)
+{
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x < y + nb && y < x + na;
 }
 
 int validate(moe_fp8_b200_handle h, const moe_fp8_b200_args* a, bool need_output = true)
@@ -574,6 +630,9 @@ int moe_fp8_b200_destroy(moe_fp8_b200_handle h)
         if (h->pipe_compute_done[i]) cudaEventDestroy(h->pipe_compute_done[i]);
         if (h->pipe_out_done[i]) cudaEventDestroy(h->pipe_out_done[i]);
     }
+    if (h->side_begin) cudaEventDestroy(h->side_begin);
+    if (h->side_done) cudaEventDestroy(h->side_done);
+    if (h->side) cudaStreamDestroy(h->side);
     if (h->pipe_in) cudaStreamDestroy(h->pipe_in);
     if (h->pipe_out) cudaStreamDestroy(h->pipe_out);
     if (h->w1_tiled) cudaFree(h->w1_tiled);
@@ -768,7 +827,7 @@ int moe_fp8_b200_finalize(moe_fp8_b200_handle h, int num_tokens, void* output, v
     if (num_tokens == 0) return MOE_FP8_B200_OK;
     if (!output || ((uintptr_t)output & 15u))
         return fail(h, MOE_FP8_B200_ERR_INVALID_ARGUMENT, "output is NULL or not 16-byte aligned");
-    const cudaError_t e = launch_combine(h->ws, output, num_tokens, static_cast<cudaStream_t>(stream));
+    const cudaError_t e = launch_combine(h->ws, output, num_tokens, 0, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "combine launch failed: %s", cudaGetErrorString(e));
     return MOE_FP8_B200_OK;
 }
@@ -832,22 +891,61 @@ int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, 
     uint8_t* d_hidden = d_logits + b_logits;
     uint8_t* d_scale = d_hidden + b_hidden;
     uint8_t* d_out = d_scale + b_scale;
-    cudaError_t e = cudaMemcpyAsync(d_logits, args->routing_logits, sizeof(float) * (size_t)T * kNumExperts,
-                                    cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_hidden, args->hidden_states, (size_t)T * hidden, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_scale, args->hidden_states_scale, sizeof(float) * hidden_blocks * T,
-                            cudaMemcpyHostToDevice, stream);
-    if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "host-to-device copy: %s", cudaGetErrorString(e));
+    const size_t n_logits = sizeof(float) * (size_t)T * kNumExperts, n_hidden = (size_t)T * hidden;
+    const size_t n_scale = sizeof(float) * hidden_blocks * T, n_out = sizeof(__nv_bfloat16) * (size_t)T * hidden;
     moe_fp8_b200_args dev = *args;
     dev.routing_logits = reinterpret_cast<const float*>(d_logits);
     dev.hidden_states = d_hidden;
     dev.hidden_states_scale = reinterpret_cast<const float*>(d_scale);
     dev.output = d_out;
+    cudaError_t e = cudaSuccess;
+    // Pinned buffers (and an output that shares no byte with an input): kernels read and write them in place, so that
+    // rows without an expert here are never brought in, their zeros leave during the GEMMs, and no copy engine's
+    // start and end lies between the kernels.  Whole call, copies / in place: 32 experts T=16 149 / 135 us, T=256
+    // 339 / 264, T=2048 1130 / 789, T=4096 2050 / 1534; 256 experts, where every row moves and a copy engine is
+    // 8 % faster than a kernel's loads and stores, T=128 1178 / 1166, T=4096 4393 / 4359.
+    const bool decode_size = T <= kDecodeMaxTokens;
+    const void *p_logits, *p_hidden, *p_scale, *p_out;
+    const bool direct = h->opt_stop_after == 0 &&
+                        pinned_range(args->routing_logits, n_logits, p_logits) &&
+                        pinned_range(args->hidden_states, n_hidden, p_hidden) &&
+                        pinned_range(args->hidden_states_scale, n_scale, p_scale) && pinned_range(args->output, n_out, p_out) &&
+                        !overlap(p_out, n_out, p_logits, n_logits) && !overlap(p_out, n_out, p_hidden, n_hidden) &&
+                        !overlap(p_out, n_out, p_scale, n_scale);
+    if (direct) {
+        const bool zero_aside = h->num_local_experts <= kZeroAsideExperts && T >= kZeroAsideTokens;
+        if (zero_aside && !h->side_done) {
+            int low = 0, high = 0;
+            e = cudaDeviceGetStreamPriorityRange(&low, &high);
+            // ahead of the combine's CTAs, which want the free SM as well
+            if (e == cudaSuccess && !h->side) e = cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, high);
+            if (e == cudaSuccess && !h->side_begin) e = cudaEventCreateWithFlags(&h->side_begin, cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->side_done, cudaEventDisableTiming);
+            if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "side stream set-up: %s", cudaGetErrorString(e));
+        }
+        FetchList list = {};
+        list.add(p_logits, d_logits, n_logits);
+        list.add(p_scale, d_scale, n_scale);
+        if (decode_size) list.add(p_hidden, d_hidden, n_hidden);
+        else dev.hidden_states = p_hidden;   // the permute reads each row that has an expert here once
+        dev.output = const_cast<void*>(p_out);
+        e = launch_fetch_inputs(list, h->num_sms, stream);
+        if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "fetch of the host inputs: %s", cudaGetErrorString(e));
+        const int rc = enqueue_layer(h, dev, stream, nullptr, true, zero_aside);
+        // a call that failed half-way leaves nothing behind that still writes to the caller's memory
+        if (rc != MOE_FP8_B200_OK && zero_aside) cudaStreamSynchronize(h->side);
+        if (rc != MOE_FP8_B200_OK) { cudaStreamSynchronize(stream); return rc; }
+        e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "host-resident call: %s", cudaGetErrorString(e));
+        return MOE_FP8_B200_OK;
+    }
+    e = cudaMemcpyAsync(d_logits, args->routing_logits, n_logits, cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_hidden, args->hidden_states, n_hidden, cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_scale, args->hidden_states_scale, n_scale, cudaMemcpyHostToDevice, stream);
+    if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "host-to-device copy: %s", cudaGetErrorString(e));
     const int rc = enqueue_layer(h, dev, stream);
     if (rc != MOE_FP8_B200_OK) return rc;
-    e = cudaMemcpyAsync(args->output, d_out, sizeof(__nv_bfloat16) * (size_t)T * hidden, cudaMemcpyDeviceToHost, stream);
+    e = cudaMemcpyAsync(args->output, d_out, n_out, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "device-to-host copy: %s", cudaGetErrorString(e));
     return MOE_FP8_B200_OK;

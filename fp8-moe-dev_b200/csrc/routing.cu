@@ -54,6 +54,7 @@ __device__ __forceinline__ void scan_tiles_block(const Workspace& ws, int num_lo
         ws.expert_offset[num_local_experts] = total * kTileM;
         ws.num_tiles[0] = total;
         ws.ctrl->blocks_done = 0;
+        ws.ctrl->permute_done = 0;
         ws.ctrl->unit_ticket[0] = ws.ctrl->unit_ticket[1] = 0;
         // the status word is sticky: the first failure stays until the host has read it
         if (overflow && atomicCAS(&ws.ctrl->status, kStatusOk, kStatusRowOverflow) == kStatusOk)
@@ -207,8 +208,13 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_dispatch_kernel(
 // ---------------------------------------------------------------------------------------
 constexpr int kPermuteWarps = 4;
 
+// `count_done`: zero_rows_kernel waits for the permute's reads of host memory; a warp that is done with them says so.
+__device__ __forceinline__ void count_permuted(const Workspace& ws, int lane, int count_done) {
+    if (count_done && lane == 0) atomicAdd(&ws.ctrl->permute_done, 1);
+}
+
 __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_kernel(
-    const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, Workspace ws, int T)
+    const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, Workspace ws, int T, int count_done)
 {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kPermuteWarps + (threadIdx.x >> 5);
@@ -224,7 +230,7 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_kernel(
         }
         ws.pair_row[(size_t)t * kTopK + lane] = r;
     }
-    if (n_pairs == 0) return;
+    if (n_pairs == 0) { count_permuted(ws, lane, count_done); return; }
 
     constexpr int kVec = kHidden / 16 / 32;  // 14 uint4 per lane
     uint4 v[kVec];
@@ -246,12 +252,12 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_kernel(
         if (lane + 32 < kHiddenBlocks) ws.sfa1[(size_t)(lane + 32) * ws.m_cap + row] = sc1;
         if (lane == 0) ws.row_token[row] = t;
     }
+    count_permuted(ws, lane, count_done);
 }
 
-// The same movement for a run-time row length (Workspace::geo.hidden, a multiple of 256 bytes): the row
-// is re-read per packed row it goes to (it sits in L1 after the first pass).
+// The same movement for a run-time row length (Workspace::geo.hidden, a multiple of 256 bytes, at most 8192).
 __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_generic_kernel(
-    const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, Workspace ws, int T)
+    const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, Workspace ws, int T, int count_done)
 {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kPermuteWarps + (threadIdx.x >> 5);
@@ -267,31 +273,40 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_generic_kerne
         }
         ws.pair_row[(size_t)t * kTopK + lane] = r;
     }
-    if (n_pairs == 0) return;
+    if (n_pairs == 0) { count_permuted(ws, lane, count_done); return; }
     const int H = ws.geo.hidden;
     const int vecs = H / 16, blocks = H / kBlock;   // <= 512 uint4, <= 64 scales
     const uint4* src = reinterpret_cast<const uint4*>(hidden + (size_t)t * H);
     const float sc0 = (lane < blocks) ? __ldg(hidden_scale + (size_t)lane * T + t) : 0.0f;
     const float sc1 = (lane + 32 < blocks) ? __ldg(hidden_scale + (size_t)(lane + 32) * T + t) : 0.0f;
+    constexpr int kMaxVec = 8192 / 16 / 32;
+    uint4 v[kMaxVec];
+#pragma unroll
+    for (int i = 0; i < kMaxVec; ++i)
+        if (lane + 32 * i < vecs) v[i] = __ldg(src + lane + 32 * i);
     for (int p = 0; p < n_pairs; ++p) {
         const uint32_t code = ws.pair_code[(size_t)t * kTopK + p];
         const int row = ws.expert_offset[code >> 24] + (int)(code & 0x00ffffffu);
         uint4* dst = reinterpret_cast<uint4*>(ws.a1 + (size_t)row * H);
-        for (int i = lane; i < vecs; i += 32) dst[i] = __ldg(src + i);
+#pragma unroll
+        for (int i = 0; i < kMaxVec; ++i)
+            if (lane + 32 * i < vecs) dst[lane + 32 * i] = v[i];
         if (lane < blocks) ws.sfa1[(size_t)lane * ws.m_cap + row] = sc0;
         if (lane + 32 < blocks) ws.sfa1[(size_t)(lane + 32) * ws.m_cap + row] = sc1;
         if (lane == 0) ws.row_token[row] = t;
     }
+    count_permuted(ws, lane, count_done);
 }
 
 // ---------------------------------------------------------------------------------------
 // Combine.  out[t, :] = bf16( sum_p float(Y[row_p, :]) * w_p ) with the pairs taken in
 // dispatch order and fp32 accumulation; tokens without a local expert get zeros.  Same
-// arithmetic as kernel/moe_fp8.cu:2276-2321.
+// arithmetic as kernel/moe_fp8.cu:2276-2321.  `out` may be pinned host memory.
 // ---------------------------------------------------------------------------------------
 constexpr int kCombineThreads = 448;  // 448 threads x 2 x 8 columns = 7168
 
-__global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, __nv_bfloat16* __restrict__ out, int T)
+__global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, __nv_bfloat16* __restrict__ out, int T,
+                                                                   int skip_empty)
 {
     const int t = blockIdx.x;
     pdl_launch_dependents();
@@ -299,6 +314,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, 
     if (t >= T) return;
     int n_pairs = ws.pair_count[t];
     if (ws.num_tiles[0] == 0) n_pairs = 0;
+    if (skip_empty && n_pairs == 0) return;   // zero_rows_kernel has that row
     float acc[2][8];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
@@ -334,7 +350,8 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, 
 }
 
 // Run-time row length: a thread walks 8-column chunks, each summed over the pairs in the same order.
-__global__ void __launch_bounds__(256) combine_generic_kernel(Workspace ws, __nv_bfloat16* __restrict__ out, int T)
+__global__ void __launch_bounds__(256) combine_generic_kernel(Workspace ws, __nv_bfloat16* __restrict__ out, int T,
+                                                              int skip_empty)
 {
     const int t = blockIdx.x;
     pdl_launch_dependents();
@@ -342,6 +359,7 @@ __global__ void __launch_bounds__(256) combine_generic_kernel(Workspace ws, __nv
     if (t >= T) return;
     int n_pairs = ws.pair_count[t];
     if (ws.num_tiles[0] == 0) n_pairs = 0;
+    if (skip_empty && n_pairs == 0) return;   // zero_rows_kernel has that row
     const int H = ws.geo.hidden;
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)t * H);
     for (int v = threadIdx.x; v < H / 8; v += blockDim.x) {
@@ -366,6 +384,64 @@ __global__ void __launch_bounds__(256) combine_generic_kernel(Workspace ws, __nv
 #pragma unroll
         for (int j = 0; j < 4; ++j) h2[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
         dst[v] = packed;
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// Host-resident calls whose buffers are pinned: the kernels reach them over PCIe themselves (see
+// moe_fp8_b200_run_host for when).
+// ---------------------------------------------------------------------------------------
+// The call's small inputs, brought to the device by one launch: what the routing kernel (logits) and the permute
+// (scales, four bytes per row and K block) read in an order that PCIe should not see, and the hidden rows where
+// every CTA of the decode kernel reads them.
+constexpr int kFetchThreads = 256, kFetchUnroll = 4;
+__global__ void __launch_bounds__(kFetchThreads) fetch_inputs_kernel(const __grid_constant__ FetchList list)
+{
+    pdl_launch_dependents();
+    pdl_wait();   // the staging may still be read by the kernels in front
+    const size_t tid = (size_t)blockIdx.x * kFetchThreads + threadIdx.x, threads = (size_t)gridDim.x * kFetchThreads;
+#pragma unroll
+    for (int k = 0; k < FetchList::kMax; ++k) {
+        if (k >= list.n) break;
+        const uint32_t* src = list.seg[k].src;
+        uint32_t* dst = list.seg[k].dst;     // 16-byte aligned
+        const size_t words = list.seg[k].words;
+        const size_t vecs = (reinterpret_cast<uintptr_t>(src) & 15u) == 0 ? words / 4 : 0;
+        for (size_t i0 = tid; i0 < vecs; i0 += threads * kFetchUnroll) {
+            uint4 v[kFetchUnroll];
+#pragma unroll
+            for (int u = 0; u < kFetchUnroll; ++u)
+                if (i0 + u * threads < vecs) v[u] = __ldg(reinterpret_cast<const uint4*>(src) + i0 + u * threads);
+#pragma unroll
+            for (int u = 0; u < kFetchUnroll; ++u)
+                if (i0 + u * threads < vecs) reinterpret_cast<uint4*>(dst)[i0 + u * threads] = v[u];
+        }
+        for (size_t i = vecs * 4 + tid; i < words; i += threads) dst[i] = __ldg(src + i);
+    }
+}
+
+// Output rows of the tokens that have no expert here (most of them where a GPU holds one shard of eight): known as
+// soon as routing is done, written to the host while the experts' GEMMs run, for which these leave one SM free.
+// Bound by PCIe, which few CTAs of plain stores fill (52 GB/s from 8 CTAs as from 296; cudaMemcpyAsync 56.7); four
+// of 512 threads fit on that one SM.  A warp per row.
+constexpr int kZeroCtas = 4, kZeroThreads = 512;
+__global__ void __launch_bounds__(kZeroThreads) zero_rows_kernel(Workspace ws, uint8_t* __restrict__ out, int T)
+{
+    const int lane = threadIdx.x & 31, warps = kZeroCtas * (kZeroThreads / 32);
+    const bool none = ws.num_tiles[0] == 0;
+    const int vecs = ws.geo.hidden * 2 / 16;
+    // Not before the permute has read its rows: its read requests would queue behind these writes on their way out
+    // (host call on 32 experts: T=512 369 us without this wait, 337 with it; T=1024 520 / 474).  Resident already,
+    // because the combine's CTAs would take the free SM.  The wait is a courtesy, nothing depends on its outcome.
+    if (threadIdx.x == 0) {
+        const uint64_t t0 = global_timer_ns();
+        while (*reinterpret_cast<volatile int*>(&ws.ctrl->permute_done) < T && global_timer_ns() - t0 < 5000000ull) __nanosleep(500);
+    }
+    __syncthreads();
+    for (int t = blockIdx.x * (kZeroThreads / 32) + (threadIdx.x >> 5); t < T; t += warps) {
+        if (!none && ws.pair_count[t] != 0) continue;
+        uint4* row = reinterpret_cast<uint4*>(out) + (size_t)t * vecs;
+        for (int i = lane; i < vecs; i += 32) row[i] = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -404,23 +480,40 @@ cudaError_t launch_route_dispatch(const float* logits, const void* bias, const W
                       do_scan);
 }
 
-cudaError_t launch_permute(const void* hidden, const float* hidden_scale, const Workspace& ws, int T,
+cudaError_t launch_permute(const void* hidden, const float* hidden_scale, const Workspace& ws, int T, int count_done,
                            cudaStream_t stream)
 {
     const int grid = (T + kPermuteWarps - 1) / kPermuteWarps;
     if (!ws.geo.is_reference())
         return launch_pdl(permute_rows_generic_kernel, dim3(grid), dim3(kPermuteWarps * 32), 0, stream,
-                          static_cast<const uint8_t*>(hidden), hidden_scale, ws, T);
+                          static_cast<const uint8_t*>(hidden), hidden_scale, ws, T, count_done);
     return launch_pdl(permute_rows_kernel, dim3(grid), dim3(kPermuteWarps * 32), 0, stream,
-                      static_cast<const uint8_t*>(hidden), hidden_scale, ws, T);
+                      static_cast<const uint8_t*>(hidden), hidden_scale, ws, T, count_done);
 }
 
-cudaError_t launch_combine(const Workspace& ws, void* out, int T, cudaStream_t stream)
+cudaError_t launch_combine(const Workspace& ws, void* out, int T, int skip_empty, cudaStream_t stream)
 {
     if (!ws.geo.is_reference())
-        return launch_pdl(combine_generic_kernel, dim3(T), dim3(256), 0, stream, ws, static_cast<__nv_bfloat16*>(out), T);
-    return launch_pdl(combine_kernel, dim3(T), dim3(kCombineThreads), 0, stream, ws, static_cast<__nv_bfloat16*>(out),
-                      T);
+        return launch_pdl(combine_generic_kernel, dim3(T), dim3(256), 0, stream, ws, static_cast<__nv_bfloat16*>(out), T,
+                          skip_empty);
+    return launch_pdl(combine_kernel, dim3(T), dim3(kCombineThreads), 0, stream, ws, static_cast<__nv_bfloat16*>(out), T,
+                      skip_empty);
+}
+
+cudaError_t launch_zero_rows(const Workspace& ws, void* out, int T, cudaStream_t stream)
+{
+    zero_rows_kernel<<<kZeroCtas, kZeroThreads, 0, stream>>>(ws, static_cast<uint8_t*>(out), T);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fetch_inputs(const FetchList& list, int num_sms, cudaStream_t stream)
+{
+    size_t words = 0;
+    for (int i = 0; i < list.n; ++i) words += list.seg[i].words;
+    const size_t per_cta = (size_t)kFetchThreads * 4 * kFetchUnroll;
+    const size_t want = (words + per_cta - 1) / per_cta;
+    const int grid = want < 1 ? 1 : want > (size_t)num_sms ? num_sms : (int)want;
+    return launch_pdl(fetch_inputs_kernel, dim3(grid), dim3(kFetchThreads), 0, stream, list);
 }
 
 
