@@ -305,6 +305,59 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_generic_kerne
 // ---------------------------------------------------------------------------------------
 constexpr int kCombineThreads = 448;  // 448 threads x 2 x 8 columns = 7168
 
+// A token's rows here and their weights: two 32-byte loads from the tables the permute kernel left behind
+// (row -1 = no such pair), one round trip instead of the chain pair count -> pair code -> expert offset.
+struct PairTable {
+    int4 row[2];
+    float4 weight[2];
+};
+__device__ __forceinline__ PairTable load_pair_table(const Workspace& ws, int t) {
+    PairTable p;
+    const int4* r = reinterpret_cast<const int4*>(ws.pair_row + (size_t)t * kTopK);
+    const float4* w = reinterpret_cast<const float4*>(ws.pair_weight + (size_t)t * kTopK);
+    p.row[0] = __ldg(r);
+    p.row[1] = __ldg(r + 1);
+    p.weight[0] = __ldg(w);
+    p.weight[1] = __ldg(w + 1);
+    return p;
+}
+
+// acc[c][0..7] += w_p * (columns 8 (v + c STRIDE) .. + 7 of row p), pair after pair; the rows of four pairs are
+// requested together.
+template <int CHUNKS, int STRIDE>
+__device__ __forceinline__ void add_rows(float (&acc)[CHUNKS][8], const __nv_bfloat16* y, int hidden, const int (&rows)[kTopK],
+                                         const float (&wts)[kTopK], int v) {
+#pragma unroll
+    for (int p0 = 0; p0 < kTopK; p0 += 4) {
+        if (rows[p0] < 0) break;   // pairs are packed from entry 0
+        uint4 raw[4][CHUNKS];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (rows[p0 + u] >= 0) {
+                const uint4* src = reinterpret_cast<const uint4*>(y + (size_t)rows[p0 + u] * hidden) + v;
+#pragma unroll
+                for (int c = 0; c < CHUNKS; ++c) raw[u][c] = __ldg(src + c * STRIDE);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (rows[p0 + u] >= 0) {
+                const float w = wts[p0 + u];
+#pragma unroll
+                for (int c = 0; c < CHUNKS; ++c) {
+                    const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw[u][c]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 f = __bfloat1622float2(h2[j]);
+                        acc[c][2 * j] += f.x * w;
+                        acc[c][2 * j + 1] += f.y * w;
+                    }
+                }
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, __nv_bfloat16* __restrict__ out, int T,
                                                                    int skip_empty)
 {
@@ -312,32 +365,18 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, 
     pdl_launch_dependents();
     pdl_wait();
     if (t >= T) return;
-    int n_pairs = ws.pair_count[t];
-    if (ws.num_tiles[0] == 0) n_pairs = 0;
-    if (skip_empty && n_pairs == 0) return;   // zero_rows_kernel has that row
+    const PairTable pairs = load_pair_table(ws, t);
+    const int rows[kTopK] = {pairs.row[0].x, pairs.row[0].y, pairs.row[0].z, pairs.row[0].w,
+                             pairs.row[1].x, pairs.row[1].y, pairs.row[1].z, pairs.row[1].w};
+    const float wts[kTopK] = {pairs.weight[0].x, pairs.weight[0].y, pairs.weight[0].z, pairs.weight[0].w,
+                              pairs.weight[1].x, pairs.weight[1].y, pairs.weight[1].z, pairs.weight[1].w};
+    if (skip_empty && rows[0] < 0) return;   // zero_rows_kernel has that row
     float acc[2][8];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[c][j] = 0.0f;
-
-    for (int p = 0; p < n_pairs; ++p) {
-        const uint32_t code = ws.pair_code[(size_t)t * kTopK + p];
-        const float w = ws.pair_weight[(size_t)t * kTopK + p];
-        const int row = ws.expert_offset[code >> 24] + (int)(code & 0x00ffffffu);
-        const uint4* src = reinterpret_cast<const uint4*>(ws.y + (size_t)row * kHidden);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const uint4 raw = __ldg(src + threadIdx.x + c * kCombineThreads);
-            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 f = __bfloat1622float2(h2[j]);
-                acc[c][2 * j] += f.x * w;
-                acc[c][2 * j + 1] += f.y * w;
-            }
-        }
-    }
+    add_rows<2, kCombineThreads>(acc, ws.y, kHidden, rows, wts, threadIdx.x);
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)t * kHidden);
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
@@ -357,32 +396,23 @@ __global__ void __launch_bounds__(256) combine_generic_kernel(Workspace ws, __nv
     pdl_launch_dependents();
     pdl_wait();
     if (t >= T) return;
-    int n_pairs = ws.pair_count[t];
-    if (ws.num_tiles[0] == 0) n_pairs = 0;
-    if (skip_empty && n_pairs == 0) return;   // zero_rows_kernel has that row
+    const PairTable pairs = load_pair_table(ws, t);
+    const int rows[kTopK] = {pairs.row[0].x, pairs.row[0].y, pairs.row[0].z, pairs.row[0].w,
+                             pairs.row[1].x, pairs.row[1].y, pairs.row[1].z, pairs.row[1].w};
+    const float wts[kTopK] = {pairs.weight[0].x, pairs.weight[0].y, pairs.weight[0].z, pairs.weight[0].w,
+                              pairs.weight[1].x, pairs.weight[1].y, pairs.weight[1].z, pairs.weight[1].w};
+    if (skip_empty && rows[0] < 0) return;   // zero_rows_kernel has that row
     const int H = ws.geo.hidden;
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)t * H);
     for (int v = threadIdx.x; v < H / 8; v += blockDim.x) {
-        float acc[8];
+        float acc[1][8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
-        for (int p = 0; p < n_pairs; ++p) {
-            const uint32_t code = ws.pair_code[(size_t)t * kTopK + p];
-            const float w = ws.pair_weight[(size_t)t * kTopK + p];
-            const int row = ws.expert_offset[code >> 24] + (int)(code & 0x00ffffffu);
-            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(ws.y + (size_t)row * H) + v);
-            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 f = __bfloat1622float2(h2[j]);
-                acc[2 * j] += f.x * w;
-                acc[2 * j + 1] += f.y * w;
-            }
-        }
+        for (int j = 0; j < 8; ++j) acc[0][j] = 0.0f;
+        add_rows<1, 0>(acc, ws.y, H, rows, wts, v);
         uint4 packed;
         __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&packed);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) h2[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
+        for (int j = 0; j < 4; ++j) h2[j] = __floats2bfloat162_rn(acc[0][2 * j], acc[0][2 * j + 1]);
         dst[v] = packed;
     }
 }
@@ -548,23 +578,6 @@ __device__ __forceinline__ uint8_t* peer_ptr(const ExchangeView& ex, int i) {
     return p;
 }
 
-// A token's rows here and their weights: two 32-byte loads from the tables the permute kernel left behind
-// (row -1 = no such pair), one round trip instead of the chain pair count -> pair code -> expert offset.
-struct PairTable {
-    int4 row[2];
-    float4 weight[2];
-};
-__device__ __forceinline__ PairTable load_pair_table(const Workspace& ws, int t) {
-    PairTable p;
-    const int4* r = reinterpret_cast<const int4*>(ws.pair_row + (size_t)t * kTopK);
-    const float4* w = reinterpret_cast<const float4*>(ws.pair_weight + (size_t)t * kTopK);
-    p.row[0] = __ldg(r);
-    p.row[1] = __ldg(r + 1);
-    p.weight[0] = __ldg(w);
-    p.weight[1] = __ldg(w + 1);
-    return p;
-}
-
 __global__ void __launch_bounds__(kCombineThreads, 2) combine_push_kernel(Workspace ws, ExchangeView ex, int T)
 {
     pdl_launch_dependents();
@@ -609,36 +622,7 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_push_kernel(Worksp
             for (int c = 0; c < 2; ++c)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) acc[c][j] = 0.0f;
-            // the rows of four pairs are requested together, then added in pair order
-#pragma unroll
-            for (int p0 = 0; p0 < kTopK; p0 += 4) {
-                if (rows[p0] < 0) break;
-                uint4 raw[4][2];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (rows[p0 + u] >= 0) {
-                        const uint4* src = reinterpret_cast<const uint4*>(ws.y + (size_t)rows[p0 + u] * kHidden);
-                        raw[u][0] = __ldg(src + threadIdx.x);
-                        raw[u][1] = __ldg(src + threadIdx.x + kCombineThreads);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (rows[p0 + u] >= 0) {
-                        const float w = wts[p0 + u];
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw[u][c]);
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const float2 f = __bfloat1622float2(h2[j]);
-                                acc[c][2 * j] += f.x * w;
-                                acc[c][2 * j + 1] += f.y * w;
-                            }
-                        }
-                    }
-                }
-            }
+            add_rows<2, kCombineThreads>(acc, ws.y, kHidden, rows, wts, threadIdx.x);
             uint4* dst = reinterpret_cast<uint4*>(dst_base + (size_t)parity * ex.rows_bytes_per_parity +
                                                   ((size_t)ex.rank * ex.slot_rows + tl) * (kHidden * 2));
 #pragma unroll
