@@ -21,8 +21,8 @@
 //     (column, token), so SwiGLU needs no exchange.  v = silu(gate) * lin goes to a small
 //     fp32 scratch (the 1x128 requantisation needs whole 128-column blocks, which span units);
 //   * phase 2 (GEMM2): a worker waits for its expert's rows in the scratch, requantises them (same arithmetic as
-//     the staged epilogue), streams 16 rows of W2 per unit the same way, and writes bf16 y rows; the first weights are requested before that wait, so the wait
-//     and the requantisation hide behind their latency;
+//     the staged epilogue), streams 16 rows of W2 per unit the same way, and writes bf16 y rows; the first
+//     weights are requested before that wait, so the wait and the requantisation hide behind their latency;
 //   * the weighted combine is a kernel of its own (decode_combine_kernel): it is resident before this one ends,
 //     so its start costs no more than a grid barrier would, and meanwhile the CTAs of the next
 //     layer's decode kernel, which need this one's shared memory, can move in.
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
     int first_ticket = 0;
     if (warp >= kDecWarps && lane == 0) first_ticket = (int)atomicAdd(&ws.ctrl->dec_ticket, 1u);
     // A failure that an earlier launch recorded stays in the status word until the host has read it
-    // (moe_fp8_b200_check clears it together with any arrival counts that launch left on the grid
-    // barriers).  Until then this kernel does nothing: with stale counts its barriers would open early.
+    // (moe_fp8_b200_check clears it; the next run then clears counter and scratch).  Until then this kernel does
+    // nothing: with a stale counter it would leave units out, with stale words phase 2 would not wait.
     // Every CTA reads the same word; within one launch it can only change after a full wait limit.
     if (__ldcg(&ws.ctrl->status) != kStatusOk) return;
     stamp(0);

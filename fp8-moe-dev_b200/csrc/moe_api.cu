@@ -1127,7 +1127,7 @@ int moe_fp8_b200_check(moe_fp8_b200_handle h, void* stream)
                     : st[0] == kStatusGemm2Timeout ? "GEMM2 gave up on a bounded wait"
                     : st[0] == kStatusRowOverflow  ? "routed rows exceed the workspace capacity"
                     : st[0] == kStatusExchangeTimeout ? "a peer rank's rows did not arrive within the wait limit"
-                    : st[0] == kStatusDecodeTimeout   ? "the decode kernel gave up on a grid barrier"
+                    : st[0] == kStatusDecodeTimeout   ? "the decode kernel gave up on a bounded wait"
                                                    : "unknown");
     return MOE_FP8_B200_OK;
 }

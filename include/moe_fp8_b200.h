@@ -200,7 +200,8 @@ MOE_FP8_B200_API int moe_fp8_b200_run(moe_fp8_b200_handle h, const moe_fp8_b200_
 
 /* Same layer with HOST pointers for the per-call tensors (routing_logits,
  * hidden_states, hidden_states_scale, output); routing_bias and the weights stay device
- * pointers.  Copies in, runs, copies out and synchronises `stream`.  This is the
+ * pointers.  Copies in, runs, copies out and synchronises `stream`; where all four lie in pinned, mapped
+ * allocations the kernels read and write them in place instead of copying.  This is the
  * end-to-end form a host-resident caller of the reference operator sees. */
 MOE_FP8_B200_API int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, void* stream);
 
@@ -346,7 +347,7 @@ MOE_FP8_B200_API int moe_fp8_b200_check(moe_fp8_b200_handle h, void* stream);
 
 /* Failure injection FROM THE HOST, for tests of the error path (nothing on the GPU faults, traps or
  * hangs): writes `status` into the device status word as if a kernel had recorded it, and
- * `stale_barrier_arrivals` into the arrival counter of the decode kernel's first grid barrier as a
+ * `stale_barrier_arrivals` into the work counter of the decode kernel as a
  * launch that gave up half-way would leave it.  Synchronises `stream`.  No counterpart in the
  * reference, whose errors go to stderr only. */
 MOE_FP8_B200_API int moe_fp8_b200_inject_device_status(moe_fp8_b200_handle h, int status,
