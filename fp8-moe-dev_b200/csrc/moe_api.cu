@@ -51,6 +51,12 @@ constexpr int kVersion = (0 << 16) | 1;
 // T=2048 789 / 1009; 64 experts: T=128 378 / 372, T=256 460 / 468, T=2048 1300 / 1384).
 constexpr int kZeroAsideExperts = 64;
 constexpr int kZeroAsideTokens = 256;
+// Half of the experts: nearly every row moves (few zero rows to leave early) and the permute and combine under which
+// transfers can hide are half as long as with all of them, so that a copy engine's 8 % higher rate wins from about
+// a thousand tokens on (copies / in place: T=1024 1291 / 1263 us, T=4096 3057 / 3055, T=8192 5504 / 5565, T=16384
+// 10145 / 10315; all 256 experts: T=4096 4267 / 4230, T=12288 10062 / 10038).
+constexpr int kHalfOfExperts = 128;
+constexpr int kHalfInPlaceTokens = 1024;
 thread_local std::string g_create_error;
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -906,7 +912,7 @@ int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, 
     // 8 % faster than a kernel's loads and stores, T=128 1178 / 1166, T=4096 4393 / 4359.
     const bool decode_size = T <= kDecodeMaxTokens;
     const void *p_logits, *p_hidden, *p_scale, *p_out;
-    const bool direct = h->opt_stop_after == 0 &&
+    const bool direct = h->opt_stop_after == 0 && (h->num_local_experts != kHalfOfExperts || T <= kHalfInPlaceTokens) &&
                         pinned_range(args->routing_logits, n_logits, p_logits) &&
                         pinned_range(args->hidden_states, n_hidden, p_hidden) &&
                         pinned_range(args->hidden_states_scale, n_scale, p_scale) && pinned_range(args->output, n_out, p_out) &&
