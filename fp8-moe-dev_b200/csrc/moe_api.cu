@@ -18,7 +18,7 @@ namespace moe {
 cudaError_t launch_route_dispatch(const float*, const void*, const Workspace&, int, int, int, float,
                                   const DispatchPolicy&, int, cudaStream_t);
 cudaError_t launch_permute(const void*, const float*, const Workspace&, int, int, cudaStream_t);
-cudaError_t launch_combine(const Workspace&, void*, int, int, cudaStream_t);
+cudaError_t launch_combine(const Workspace&, void*, int, int, int, cudaStream_t);
 cudaError_t launch_zero_rows(const Workspace&, void*, int, cudaStream_t);
 cudaError_t launch_fetch_inputs(const FetchList&, int, cudaStream_t);
 cudaError_t launch_quantize_rows(const void*, void*, float*, int, int, cudaStream_t);
@@ -384,7 +384,7 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
             e = launch_combine_push(h->ws, *ex, T, stream);
             if (e == cudaSuccess) e = launch_reduce_owned(h->ws, *ex, T, a.output, stream);
         } else {
-            e = launch_combine(h->ws, a.output, T, zero_aside ? 1 : 0, stream);
+            e = launch_combine(h->ws, a.output, T, zero_aside ? 1 : 0, /*from_views=*/0, stream);
         }
     }
     if (e == cudaSuccess && zero_aside) e = cudaStreamWaitEvent(stream, h->side_done, 0);
@@ -833,7 +833,7 @@ int moe_fp8_b200_finalize(moe_fp8_b200_handle h, int num_tokens, void* output, v
     if (num_tokens == 0) return MOE_FP8_B200_OK;
     if (!output || ((uintptr_t)output & 15u))
         return fail(h, MOE_FP8_B200_ERR_INVALID_ARGUMENT, "output is NULL or not 16-byte aligned");
-    const cudaError_t e = launch_combine(h->ws, output, num_tokens, 0, static_cast<cudaStream_t>(stream));
+    const cudaError_t e = launch_combine(h->ws, output, num_tokens, 0, /*from_views=*/1, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "combine launch failed: %s", cudaGetErrorString(e));
     return MOE_FP8_B200_OK;
 }

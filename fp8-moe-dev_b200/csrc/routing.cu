@@ -321,6 +321,27 @@ __device__ __forceinline__ PairTable load_pair_table(const Workspace& ws, int t)
     p.weight[1] = __ldg(w + 1);
     return p;
 }
+// The same table from what moe_fp8_b200_run_unfinalized publishes (pair count, pair code, expert offset): those are
+// what finalize combines, also where the caller has changed them since.
+__device__ __forceinline__ PairTable pair_table_from_views(const Workspace& ws, int t) {
+    const int n_pairs = ws.num_tiles[0] == 0 ? 0 : ws.pair_count[t];
+    const float4* w = reinterpret_cast<const float4*>(ws.pair_weight + (size_t)t * kTopK);
+    int r[kTopK];
+#pragma unroll
+    for (int p = 0; p < kTopK; ++p) {
+        r[p] = -1;
+        if (p < n_pairs) {
+            const uint32_t code = ws.pair_code[(size_t)t * kTopK + p];
+            r[p] = ws.expert_offset[code >> 24] + (int)(code & 0x00ffffffu);
+        }
+    }
+    PairTable t8;
+    t8.row[0] = make_int4(r[0], r[1], r[2], r[3]);
+    t8.row[1] = make_int4(r[4], r[5], r[6], r[7]);
+    t8.weight[0] = w[0];
+    t8.weight[1] = w[1];
+    return t8;
+}
 
 // acc[c][0..7] += w_p * (columns 8 (v + c STRIDE) .. + 7 of row p), pair after pair; the rows of four pairs are
 // requested together.
@@ -358,6 +379,8 @@ __device__ __forceinline__ void add_rows(float (&acc)[CHUNKS][8], const __nv_bfl
     }
 }
 
+// VIEWS: the token's rows come from the published tables (finalize) instead of the permute's.
+template <bool VIEWS>
 __global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, __nv_bfloat16* __restrict__ out, int T,
                                                                    int skip_empty)
 {
@@ -365,7 +388,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, 
     pdl_launch_dependents();
     pdl_wait();
     if (t >= T) return;
-    const PairTable pairs = load_pair_table(ws, t);
+    const PairTable pairs = VIEWS ? pair_table_from_views(ws, t) : load_pair_table(ws, t);
     const int rows[kTopK] = {pairs.row[0].x, pairs.row[0].y, pairs.row[0].z, pairs.row[0].w,
                              pairs.row[1].x, pairs.row[1].y, pairs.row[1].z, pairs.row[1].w};
     const float wts[kTopK] = {pairs.weight[0].x, pairs.weight[0].y, pairs.weight[0].z, pairs.weight[0].w,
@@ -389,6 +412,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, 
 }
 
 // Run-time row length: a thread walks 8-column chunks, each summed over the pairs in the same order.
+template <bool VIEWS>
 __global__ void __launch_bounds__(256) combine_generic_kernel(Workspace ws, __nv_bfloat16* __restrict__ out, int T,
                                                               int skip_empty)
 {
@@ -396,7 +420,7 @@ __global__ void __launch_bounds__(256) combine_generic_kernel(Workspace ws, __nv
     pdl_launch_dependents();
     pdl_wait();
     if (t >= T) return;
-    const PairTable pairs = load_pair_table(ws, t);
+    const PairTable pairs = VIEWS ? pair_table_from_views(ws, t) : load_pair_table(ws, t);
     const int rows[kTopK] = {pairs.row[0].x, pairs.row[0].y, pairs.row[0].z, pairs.row[0].w,
                              pairs.row[1].x, pairs.row[1].y, pairs.row[1].z, pairs.row[1].w};
     const float wts[kTopK] = {pairs.weight[0].x, pairs.weight[0].y, pairs.weight[0].z, pairs.weight[0].w,
@@ -521,13 +545,14 @@ cudaError_t launch_permute(const void* hidden, const float* hidden_scale, const 
                       static_cast<const uint8_t*>(hidden), hidden_scale, ws, T, count_done);
 }
 
-cudaError_t launch_combine(const Workspace& ws, void* out, int T, int skip_empty, cudaStream_t stream)
+cudaError_t launch_combine(const Workspace& ws, void* out, int T, int skip_empty, int from_views, cudaStream_t stream)
 {
+    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
     if (!ws.geo.is_reference())
-        return launch_pdl(combine_generic_kernel, dim3(T), dim3(256), 0, stream, ws, static_cast<__nv_bfloat16*>(out), T,
-                          skip_empty);
-    return launch_pdl(combine_kernel, dim3(T), dim3(kCombineThreads), 0, stream, ws, static_cast<__nv_bfloat16*>(out), T,
-                      skip_empty);
+        return launch_pdl(from_views ? combine_generic_kernel<true> : combine_generic_kernel<false>, dim3(T), dim3(256), 0, stream,
+                          ws, o, T, skip_empty);
+    return launch_pdl(from_views ? combine_kernel<true> : combine_kernel<false>, dim3(T), dim3(kCombineThreads), 0, stream, ws, o,
+                      T, skip_empty);
 }
 
 cudaError_t launch_zero_rows(const Workspace& ws, void* out, int T, cudaStream_t stream)

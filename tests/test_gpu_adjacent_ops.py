@@ -109,6 +109,44 @@ def test_unfinalized_plus_finalize_equals_run(pkg, layer32, T, offset):
     assert torch.equal(out.cpu(), want)
 
 
+@pytest.mark.parametrize("T,hidden,inter", [(1, 7168, 2048), (40, 7168, 2048), (300, 7168, 2048), (40, 1024, 512)])
+def test_finalize_combines_the_published_tables(pkg, T, hidden, inter):
+    """What a caller changes in the views between run_unfinalized and finalize takes effect: a dropped pair, two
+    pairs in the other order, a row taken from another slot, another weight."""
+    from fp8_moe_dev_b200 import gen
+    layer = pkg.MoeLayer(T, 256, 0, hidden=hidden, intermediate=inter)   # all experts: every token has pairs
+    try:
+        logits, bias = gen.make_routing(T, seed=940 + T)
+        hid, scale = gen.make_hidden(T, seed=941 + T, hidden=hidden)
+        weights = gen.make_shard(0, 256, device="cuda", out_device="cuda", hidden=hidden, inter=inter)
+        v = layer.run_unfinalized(logits.cuda(), bias.cuda(), hid.cuda(), scale.cuda(), *weights, 0, RSF)
+        layer.check()
+        cnt, code, wt = v["pair_count"], v["pair_code"], v["pair_weight"]
+        assert int(cnt.min()) >= 2
+        cnt[0::3] -= 1                                  # the last pair of every third token is left out
+        swap = code[:, 0].clone()
+        code[:, 0] = code[:, 1]
+        code[:, 1] = swap
+        swap = wt[:, 0].clone()
+        wt[:, 0] = wt[:, 1]
+        wt[:, 1] = swap * 0.5                           # ... and the former first pair counts half
+        if T > 1:
+            code[1, 0] = code[T - 1, 0]                 # one token takes another one's row
+        off = v["expert_offset"].long()
+        rows = off[(code.long() & 0xFFFFFFFF) >> 24] + (code.long() & 0xFFFFFF)
+        live = torch.arange(8, device="cuda")[None, :] < cnt[:, None]
+        terms = v["y"][torch.where(live, rows, 0)].double() * torch.where(live, wt, 0.0).double()[:, :, None]
+        want, mag = terms.sum(1), terms.abs().sum(1)
+        out = torch.empty(T, hidden, dtype=torch.bfloat16, device="cuda")
+        layer.finalize(T, out)
+        layer.check()
+        # bf16 rounding of the result, eight fp32 roundings of the partial sums
+        err = (out.double() - want).abs()
+        assert bool((err <= 2.0 ** -8 * want.abs() + 8 * 2.0 ** -24 * mag + 1e-30).all())
+    finally:
+        layer.close()
+
+
 def test_quantize_hidden_every_bf16_maximum(pkg, oracle, layer32):
     """Every positive finite bf16 value (subnormals included) as a block maximum: the scale
     amax / 448 and the payloads must match the oracle's divisions bit for bit."""
