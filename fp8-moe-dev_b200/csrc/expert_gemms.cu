@@ -133,8 +133,8 @@ template <bool GENERIC, bool SMALLA>
 __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
     const __grid_constant__ CUtensorMap tmap_a1, const __grid_constant__ CUtensorMap tmap_w1,
     const __grid_constant__ CUtensorMap tmap_a2, const __grid_constant__ CUtensorMap tmap_w2,
-    const __grid_constant__ CUtensorMap tmap_y, Workspace ws, const float2* __restrict__ w1_scale,
-    const float2* __restrict__ w2_scale, int silu_exact, int phases)
+    const __grid_constant__ CUtensorMap tmap_y, Workspace ws, const float* __restrict__ w1_scale,
+    const float* __restrict__ w2_scale, int silu_exact, int phases)
 {
     static_assert(!(SMALLA && GENERIC), "the 64-row activation box is a variant of the reference's geometry");
     const int hidden = GENERIC ? ws.geo.hidden : kHidden;
@@ -466,13 +466,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
             const bool g1 = d.mode == 1;
             const int kblocks = g1 ? kb_gemm1 : kb_gemm2;
             const float* sfa = (g1 ? ws.sfa1 : ws.sfa2) + d.row0 + row;
-            // The tile's weight-block scales for all K blocks, from the pre-laid-out copy (one float2 per
-            // K block, see repack_weight_scales_kernel): lane l keeps the entries of K blocks l and l + 32,
+            // The tile's weight-block scales for all K blocks: lane l keeps the entries of K blocks l and l + 32,
             // a K block's pair then comes from a shuffle instead of two dependent global loads.
-            const float2* sw_tile = g1 ? w1_scale + ((size_t)d.e * tiles_n1 + d.n) * kb_gemm1
-                                       : w2_scale + ((size_t)d.e * tiles_n2 + d.n) * kb_gemm2;
-            const float2 sw_a = (lane < kblocks) ? __ldg(sw_tile + lane) : make_float2(0.0f, 0.0f);
-            const float2 sw_b = (lane + 32 < kblocks) ? __ldg(sw_tile + lane + 32) : make_float2(0.0f, 0.0f);
+            const ScaleRows sw = weight_scale_rows(g1 ? w1_scale : w2_scale, ws.scales_in_place != 0, g1, d.e, d.n,
+                                                   g1 ? tiles_n1 : tiles_n2, kblocks);
+            const float2 sw_a = (lane < kblocks) ? sw.at(lane) : make_float2(0.0f, 0.0f);
+            const float2 sw_b = (lane + 32 < kblocks) ? sw.at(lane + 32) : make_float2(0.0f, 0.0f);
             // .x scales the tile's first 128-column block (GEMM1: linear branch), .y its second (gated branch)
             float acc[128];
 #pragma unroll
@@ -530,18 +529,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
             if (warp_has_rows) {
                 uint8_t* ra = tile_stage + h * kPanelBytes + row * 128;
                 uint8_t* rb = tile_stage + (2 + h) * kPanelBytes + row * 128;
-                const uint32_t sw = (uint32_t)(row & 7);
+                const uint32_t swz = (uint32_t)(row & 7);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     uint4 pk;
                     __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) h2[i] = __floats2bfloat162_rn(acc[8 * c + 2 * i], acc[8 * c + 2 * i + 1]);
-                    *reinterpret_cast<uint4*>(ra + (((uint32_t)c ^ sw) << 4)) = pk;
+                    *reinterpret_cast<uint4*>(ra + (((uint32_t)c ^ swz) << 4)) = pk;
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         h2[i] = __floats2bfloat162_rn(acc[64 + 8 * c + 2 * i], acc[64 + 8 * c + 2 * i + 1]);
-                    *reinterpret_cast<uint4*>(rb + (((uint32_t)c ^ sw) << 4)) = pk;
+                    *reinterpret_cast<uint4*>(rb + (((uint32_t)c ^ swz) << 4)) = pk;
                 }
                 if (!g1) fence_proxy_async_smem();   // the TMA stores read these writes
             }
@@ -591,8 +590,7 @@ cudaError_t launch_expert_gemms(const GemmMaps& maps, const Workspace& ws, const
     auto map = [](const void* p) { return *static_cast<const CUtensorMap*>(p); };
     auto go = [&](auto* kernel) {
         return cudaLaunchKernelEx(&cfg, kernel, map(maps.a1), map(maps.w1), map(maps.a2), map(maps.w2), map(maps.y), ws,
-                                  reinterpret_cast<const float2*>(w1_scale), reinterpret_cast<const float2*>(w2_scale), silu_exact,
-                                  phases);
+                                  w1_scale, w2_scale, silu_exact, phases);
     };
     if (!ws.geo.is_reference()) return go(expert_gemms_kernel<true, false>);
     return small_a ? go(expert_gemms_kernel<false, true>) : go(expert_gemms_kernel<false, false>);

@@ -130,7 +130,7 @@ __device__ __forceinline__ float round_bf16(float x) {
 template <int MODE>
 __global__ void __launch_bounds__(kGemmThreads, 1) splitk_gemm_kernel(
     const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, Workspace ws,
-    const float2* __restrict__ w_scale_packed, int silu_exact)
+    const float* __restrict__ w_scale, int silu_exact)
 {
     constexpr int hidden = kHidden, inter = kInter;
     constexpr int kKBlocks = ((MODE == 1) ? hidden : inter) / kBlock;               // 56 / 16
@@ -289,12 +289,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) splitk_gemm_kernel(
             unit_range(kKBlocks, u % plan.split, plan.split, kb0, kb1);
             const int grow = tc.row0 + row;
             const float* sfa = ((MODE == 1) ? ws.sfa1 : ws.sfa2) + grow;
-            // The tile's weight-block scales for all K blocks, from the pre-laid-out copy (one float2 per
-            // K block, see repack_weight_scales_kernel): lane l keeps the entries of K blocks l and l + 32,
+            // The tile's weight-block scales for all K blocks: lane l keeps the entries of K blocks l and l + 32,
             // a K block's pair then comes from a shuffle instead of two dependent global loads.
-            const float2* sw_tile = w_scale_packed + ((size_t)tc.e * kTilesN + tc.n) * kKBlocks;
-            const float2 sw_a = (lane < kKBlocks) ? __ldg(sw_tile + lane) : make_float2(0.0f, 0.0f);
-            const float2 sw_b = (kKBlocks > 32 && lane + 32 < kKBlocks) ? __ldg(sw_tile + lane + 32) : make_float2(0.0f, 0.0f);
+            const ScaleRows sw = weight_scale_rows(w_scale, ws.scales_in_place != 0, MODE == 1, tc.e, tc.n, kTilesN, kKBlocks);
+            const float2 sw_a = (lane < kKBlocks) ? sw.at(lane) : make_float2(0.0f, 0.0f);
+            const float2 sw_b = (kKBlocks > 32 && lane + 32 < kKBlocks) ? sw.at(lane + 32) : make_float2(0.0f, 0.0f);
             // .x scales the tile's first 128-column block (GEMM1: linear branch), .y its second (gated branch)
             const float mine_a = sw_a.x, other_a = sw_a.y;
             const float mine_b = sw_b.x, other_b = sw_b.y;
@@ -473,7 +472,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) splitk_gemm_kernel(
 
 // ---------------------------------------------------------------------------------------
 // Weight-scale pre-layout, run once per pair of scale tensors (the handle remembers their
-// addresses): the promotion wants, per output tile and K block, the two 128x128-block scales the
+// addresses; not used where the scales are read in place): the promotion wants, per output tile and K block, the two 128x128-block scales the
 // tile's 256 accumulator columns use.  In the operator's layout those lie kInterBlocks rows apart
 // (GEMM1: [E, 32, 56], linear-branch block n and gated-branch block 16 + n) or in neighbouring
 // rows (GEMM2: [E, 56, 16], blocks 2n and 2n + 1); here they become one float2 per (expert, tile,
@@ -653,10 +652,9 @@ cudaError_t configure_gemm_kernels()
     return e;
 }
 
-cudaError_t launch_splitk_gemm(int mode, const GemmMaps& maps, const Workspace& ws, const float* w_scale_packed, int silu_exact,
+cudaError_t launch_splitk_gemm(int mode, const GemmMaps& maps, const Workspace& ws, const float* w_scale, int silu_exact,
                                int num_ctas, cudaStream_t stream)
 {
-    const float2* w_scale = reinterpret_cast<const float2*>(w_scale_packed);
     const CUtensorMap* ma = static_cast<const CUtensorMap*>(mode == 1 ? maps.a1 : maps.a2);
     const CUtensorMap* mb = static_cast<const CUtensorMap*>(mode == 1 ? maps.w1 : maps.w2);
     cudaLaunchConfig_t cfg = {};

@@ -31,6 +31,31 @@ struct TileCoord {
     int e, n, row0, rows;
 };
 
+// Where the two weight-block scales of an output tile lie, K block after K block: .lo scales its first 128 columns
+// (GEMM1: linear branch), .hi its second (gated branch).  In the handle's copy (repack_weight_scales_kernel) a
+// K block's two lie side by side; in the operator's own layout, where both tensors have 2 tiles_n rows per expert,
+// they are two rows contiguous in the K block: n and tiles_n + n of GEMM1's tensor, 2n and 2n + 1 of GEMM2's.  A
+// warp reads a unit's scales once, ahead of its K loop, so either form serves.
+struct ScaleRows {
+    const float *lo, *hi;
+    int step;
+    __device__ __forceinline__ float2 at(int kb) const { return make_float2(__ldg(lo + kb * step), __ldg(hi + kb * step)); }
+};
+__device__ __forceinline__ ScaleRows weight_scale_rows(const float* base, bool in_place, bool gemm1, int e, int n, int tiles_n,
+                                                       int kblocks) {
+    ScaleRows r;
+    if (in_place) {
+        r.lo = base + ((size_t)e * 2 * tiles_n + (gemm1 ? n : 2 * n)) * kblocks;
+        r.hi = r.lo + (size_t)(gemm1 ? tiles_n : 1) * kblocks;
+        r.step = 1;
+    } else {
+        r.lo = base + ((size_t)e * tiles_n + n) * kblocks * 2;
+        r.hi = r.lo + 1;
+        r.step = 2;
+    }
+    return r;
+}
+
 // tcgen05.wait::ld with the destination registers as in/out operands, so that the
 // compiler cannot move a use of them above the wait.
 __device__ __forceinline__ void tmem_ld_wait2(uint32_t (&a)[32], uint32_t (&b)[32]) {

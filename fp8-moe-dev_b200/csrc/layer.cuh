@@ -149,6 +149,7 @@ struct Workspace {
     int m_cap;              // packed-row capacity (multiple of 128)
     int max_tiles;
     Geometry geo;
+    int scales_in_place;    // the GEMMs' weight scales are the operator's own tensors, not the handle's copy
     int w_tiled;            // the GEMMs' weight map covers the tile-ordered copy (one 32 KB piece per tile and K block)
 };
 

@@ -169,6 +169,7 @@ struct moe_fp8_b200_ctx {
     float* sw2_packed = nullptr;
     const float* cached_s1 = nullptr;
     const float* cached_s2 = nullptr;
+    int opt_scales_in_place = 0;   // MOE_FP8_B200_OPT_SCALES_IN_PLACE: no such copy
     // optional per-stage timing: events around each stage of the last kTimedRuns runs
     int opt_stage_timing = 0;
     static constexpr int kTimedRuns = 64;
@@ -320,7 +321,8 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
         }
         return MOE_FP8_B200_OK;
     }
-    if (e == cudaSuccess && (a.gemm1_weights_scale != h->cached_s1 || a.gemm2_weights_scale != h->cached_s2)) {
+    const bool in_place = h->opt_scales_in_place != 0;
+    if (e == cudaSuccess && !in_place && (a.gemm1_weights_scale != h->cached_s1 || a.gemm2_weights_scale != h->cached_s2)) {
         // new scale tensors: lay them out for the GEMMs' promotion (stream-ordered in front of the chain)
         e = launch_repack_weight_scales(a.gemm1_weights_scale, a.gemm2_weights_scale, h->sw1_packed, h->sw2_packed, E, h->geo,
                                         stream);
@@ -337,6 +339,9 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
     }
     Workspace gemm_ws = h->ws;
     gemm_ws.w_tiled = tiled ? 1 : 0;
+    gemm_ws.scales_in_place = in_place ? 1 : 0;
+    const float* scale1 = in_place ? a.gemm1_weights_scale : h->sw1_packed;
+    const float* scale2 = in_place ? a.gemm2_weights_scale : h->sw2_packed;
     mark(0);
     if (e == cudaSuccess)
         e = launch_route_dispatch(a.routing_logits, a.routing_bias, h->ws, T, (int)a.local_expert_offset, E,
@@ -363,13 +368,13 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
     // runs); CTAs without work leave at once
     const int gemm_ctas = zero_aside && h->num_sms > 1 ? h->num_sms - 1 : h->num_sms;
     auto gemms = [&](int phases) {
-        return launch_expert_gemms(maps, gemm_ws, h->sw1_packed, h->sw2_packed, h->opt_exact_silu, phases, gemm_ctas, small_a, stream);
+        return launch_expert_gemms(maps, gemm_ws, scale1, scale2, h->opt_exact_silu, phases, gemm_ctas, small_a, stream);
     };
     if (split_k) {
         if (e == cudaSuccess && stop >= 3)
-            e = launch_splitk_gemm(1, maps, gemm_ws, h->sw1_packed, h->opt_exact_silu, h->num_sms, stream);
+            e = launch_splitk_gemm(1, maps, gemm_ws, scale1, h->opt_exact_silu, h->num_sms, stream);
         mark(4);
-        if (e == cudaSuccess && stop >= 4) e = launch_splitk_gemm(2, maps, gemm_ws, h->sw2_packed, 0, h->num_sms, stream);
+        if (e == cudaSuccess && stop >= 4) e = launch_splitk_gemm(2, maps, gemm_ws, scale2, 0, h->num_sms, stream);
     } else if (ev || stop == 3) {
         // the same kernel cut between the two GEMMs, for callers that time or read what lies between them
         if (e == cudaSuccess && stop >= 3) e = gemms(1);
@@ -670,6 +675,7 @@ int moe_fp8_b200_set_option(moe_fp8_b200_handle h, int option, int value)
             h->opt_wait_limit_us = value;
             return MOE_FP8_B200_OK;
         case MOE_FP8_B200_OPT_SMALL_BATCH_RING: h->opt_small_batch_ring = value ? 1 : 0; return MOE_FP8_B200_OK;
+        case MOE_FP8_B200_OPT_SCALES_IN_PLACE: h->opt_scales_in_place = value ? 1 : 0; return MOE_FP8_B200_OK;
         case MOE_FP8_B200_OPT_WEIGHT_PRELAYOUT: {
             const int on = value ? 1 : 0;
             if (on == h->opt_weight_prelayout) return MOE_FP8_B200_OK;

@@ -8,8 +8,8 @@
 //     through TVM-FFI (the reference checks nothing, kernel/moe_fp8.cu:2671-2672);
 //   * work is enqueued on the TVM-FFI environment stream of the tensors' device (the
 //     reference always uses the legacy default stream, kernel/moe_fp8.cu:2691);
-//   * nothing is cached by pointer identity, so changed tensor contents are always seen
-//     (the reference replays cached routing and graphs, kernel/moe_fp8.cu:2696-2702).
+//   * no tensor's contents are remembered from call to call (TMA descriptors are, which hold
+//     addresses only), so changed contents are always seen (the reference replays cached routing and graphs, kernel/moe_fp8.cu:2696-2702).
 // The workspace is one grow-only handle per host thread, device and expert count, as in
 // kernel/moe_fp8.cu:2677-2689.
 #include <tvm/ffi/container/tensor.h>
@@ -76,6 +76,8 @@ void run(ffi::TensorView routing_logits, ffi::TensorView routing_bias, ffi::Tens
         if (moe_fp8_b200_create(&slot.h, device, cap, (int)E) != MOE_FP8_B200_OK)
             TVM_FFI_THROW(RuntimeError) << "moe_fp8_b200_create: " << moe_fp8_b200_last_error(nullptr);
         slot.capacity = cap;
+        // this entry point's callers have nothing to invalidate a copy of the scales with
+        moe_fp8_b200_set_option(slot.h, MOE_FP8_B200_OPT_SCALES_IN_PLACE, 1);
     }
     moe_fp8_b200_args a;
     a.routing_logits = static_cast<const float*>(ptr(routing_logits));

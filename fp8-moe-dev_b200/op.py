@@ -135,6 +135,13 @@ class MoeLayer:
         if rc != _lib.OK:
             self._raise(rc)
 
+    def set_scales_in_place(self, on: bool):
+        """The GEMMs read the weight scales from the tensors of each call (nothing to invalidate) instead of a copy
+        remembered by address (default)."""
+        rc = self._lib.moe_fp8_b200_set_option(self._h, _lib.OPT_SCALES_IN_PLACE, int(bool(on)))
+        if rc != _lib.OK:
+            self._raise(rc)
+
     def inject_device_status(self, status: int, stale_barrier_arrivals: int = 0):
         """Host-side failure injection for tests of the error path (see the header)."""
         stream = torch.cuda.current_stream(self.device).cuda_stream
@@ -421,6 +428,7 @@ def run(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_
         if layer is not None:
             layer.close()
         layer = MoeLayer(max(T, 16), E, dev)
+        layer.set_scales_in_place(True)   # a caller of this function has nothing to invalidate a copy with
         _layers[key] = layer
     layer.run(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights, gemm1_weights_scale,
               gemm2_weights, gemm2_weights_scale, local_expert_offset, routed_scaling_factor, output)

@@ -110,7 +110,12 @@ enum {
     /* Batches of 5 to 64 tokens (reference geometry): the GEMMs load 64-row activation boxes (an expert cannot
      * have more rows) and use the room for a fourth operand stage, i.e. more weight bytes in flight per SM
      * (default 1).  0 = the three-stage kernel of the larger batches.  Bit-identical results. */
-    MOE_FP8_B200_OPT_SMALL_BATCH_RING = 9
+    MOE_FP8_B200_OPT_SMALL_BATCH_RING = 9,
+    /* 1: the GEMMs read the weight scales from the caller's tensors on every run instead of the handle's copy, which
+     * is remembered by address (moe_fp8_b200_invalidate_weights): other contents under the same addresses are seen
+     * without a word.  What a caller needs that has no handle to invalidate; the drop-in entry points set it.
+     * Bit-identical results.  Default 0. */
+    MOE_FP8_B200_OPT_SCALES_IN_PLACE = 10
 };
 #define MOE_FP8_B200_DECODE_MAX_TOKENS 8
 
@@ -293,7 +298,8 @@ MOE_FP8_B200_API int moe_fp8_b200_run_reduce_scatter(moe_fp8_b200_handle h, cons
  * the GEMMs' accumulator promotion walks them (one pair of block scales per output tile and K block).
  * A run whose weight or scale pointers differ from the remembered ones redoes that step in front of
  * its kernels, stream-ordered.  If the CONTENTS of the scale tensors change under the same addresses
- * (weights reloaded in place), call this before the next run.  The reference keeps the same kind of
+ * (weights reloaded in place), call this before the next run, or set MOE_FP8_B200_OPT_SCALES_IN_PLACE,
+ * which keeps no copy.  The reference keeps the same kind of
  * pointer-keyed cache for its transposed weight scales (kernel/moe_fp8.cu:3007-3014, 3501-3508) and has
  * no way to invalidate it; its activations-side caches have no counterpart here. */
 MOE_FP8_B200_API int moe_fp8_b200_invalidate_weights(moe_fp8_b200_handle h);
