@@ -11,7 +11,7 @@
 //   * no tensor's contents are remembered from call to call (TMA descriptors are, which hold
 //     addresses only), so changed contents are always seen (the reference replays cached routing and graphs, kernel/moe_fp8.cu:2696-2702).
 // The workspace is one grow-only handle per host thread, device and expert count, as in
-// kernel/moe_fp8.cu:2677-2689.
+// kernel/moe_fp8.cu:2677-2689; a thread that changes its stream orders the two itself.
 #include <tvm/ffi/container/tensor.h>
 #include <tvm/ffi/extra/c_env_api.h>
 #include <tvm/ffi/function.h>

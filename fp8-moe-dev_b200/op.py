@@ -9,6 +9,7 @@ the current stream; all compute happens in libmoe_fp8_b200.so.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import Dict, Optional, Tuple
 
 import numpy as np
@@ -385,8 +386,6 @@ class MoeLayer:
 
 
 # ----------------------------------------------------------------------------------------
-# The reference-shaped entry point: one grow-only handle per (device, expert count), like
-# the reference's thread-local workspace (kernel/moe_fp8.cu:2677-2689).
 def expert_loads(routing_logits, routing_bias, routed_scaling_factor: float = 1.0, reference_pruning: bool = True):
     """Routed rows per global expert (256 counts, a CPU list) for the first <= 4096 tokens of a
     batch: the calibration input of the load-aware expert placement.  Runs the library's routing
@@ -411,25 +410,74 @@ def expert_loads(routing_logits, routing_bias, routed_scaling_factor: float = 1.
         return [int(x) for x in cnt.cpu().tolist()]
 
 
-_layers: Dict[Tuple[int, int], MoeLayer] = {}
+# ----------------------------------------------------------------------------------------
+# The reference-shaped entry point: one grow-only handle per (device, expert count), like the
+# reference's workspace (kernel/moe_fp8.cu:2677-2689), shared by the process: a handle per thread
+# would cost its workspace each (3 GB for 16384 tokens on 32 experts).
+class _Shared:
+    """A handle and the stream that carries its latest call.  Calls on it take turns: threads under `_lock`
+    (a call only enqueues), streams by an event, since every call writes the same workspace."""
+    __slots__ = ("layer", "raw", "stream", "foreign", "done")
+
+    def __init__(self, layer):
+        self.layer, self.raw, self.stream, self.foreign, self.done = layer, None, None, False, None
+
+    def take_over(self, raw, stream):
+        """The current stream, not the one of the latest call, is to run behind that call.  Not inside a stream
+        capture: what a graph is replayed behind is up to whoever replays it."""
+        prev = self.stream
+        if prev is not None and not _capturing(stream):
+            if self.foreign:
+                if self.done is not None:
+                    stream.wait_event(self.done)
+            elif not _capturing(prev):
+                stream.wait_stream(prev)
+        self.raw, self.stream, self.done = raw, stream, None
+        # a stream id is 0 for the default stream, odd for torch's own ones, the (even) handle for a foreign one
+        self.foreign = stream.stream_id != 0 and stream.stream_id & 1 == 0
+
+    def handed_out(self):
+        """A call is enqueued on a foreign stream, which its owner may destroy at any time: its event is recorded
+        now.  Torch's own streams live as long as the process, so theirs can wait until another stream comes."""
+        if not _capturing(self.stream):
+            self.done = self.stream.record_event()
+
+
+def _capturing(stream) -> bool:
+    with torch.cuda.stream(stream):
+        return torch.cuda.is_current_stream_capturing()
+
+
+_raw_stream = torch._C._cuda_getCurrentRawStream   # the handle alone: no Stream object on every call
+_layers: Dict[Tuple[int, int], _Shared] = {}
+_lock = threading.Lock()
 
 
 def run(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights, gemm1_weights_scale,
         gemm2_weights, gemm2_weights_scale, local_expert_offset, routed_scaling_factor, output):
-    """Drop-in for the reference's `run` (destination passing, returns None)."""
+    """Drop-in for the reference's `run` (destination passing, returns None).  May be called from any thread and
+    stream: calls that share a device and expert count run one after the other."""
     T = int(routing_logits.shape[0])
     if T <= 0:
         return None
     dev = routing_logits.device.index if routing_logits.is_cuda else torch.cuda.current_device()
     E = int(gemm1_weights.shape[0])
     key = (dev, E)
-    layer = _layers.get(key)
-    if layer is None or layer.max_tokens < T:
-        if layer is not None:
-            layer.close()
-        layer = MoeLayer(max(T, 16), E, dev)
-        layer.set_scales_in_place(True)   # a caller of this function has nothing to invalidate a copy with
-        _layers[key] = layer
-    layer.run(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights, gemm1_weights_scale,
-              gemm2_weights, gemm2_weights_scale, local_expert_offset, routed_scaling_factor, output)
+    raw = _raw_stream(dev)
+    with _lock:
+        shared = _layers.get(key)
+        if shared is None or shared.layer.max_tokens < T:
+            if shared is not None:
+                del _layers[key]
+                shared.layer.close()   # waits for the device
+            layer = MoeLayer(max(T, 16), E, dev)
+            layer.set_scales_in_place(True)   # a caller of this function has nothing to invalidate a copy with
+            shared = _layers[key] = _Shared(layer)
+        if raw != shared.raw:
+            shared.take_over(raw, torch.cuda.current_stream(dev))
+        shared.layer.run(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights, gemm1_weights_scale,
+                         gemm2_weights, gemm2_weights_scale, local_expert_offset, routed_scaling_factor, output,
+                         stream=raw)
+        if shared.foreign:
+            shared.handed_out()
     return None

@@ -1,4 +1,6 @@
 """The drop-in `run(...)`, whose handles the caller never sees: what it may not remember from one call to the next."""
+import threading
+
 import pytest
 import torch
 
@@ -58,3 +60,37 @@ def test_scales_in_place_change_nothing(pkg, T, E, hidden, inter, decode):
         assert torch.equal(outs[1], outs[0]) and torch.equal(outs[2], outs[0])
     finally:
         layer.close()
+
+
+def test_overlapping_calls_from_threads_and_streams(pkg):
+    """Calls of several batch sizes on two threads, each with a stream of its own and one made outside torch, none of
+    them ordered by the caller: every result is the one of a call alone."""
+    cases = {}
+    for T in (3, 40, 300):
+        dev = [x.cuda() for x in hp.cpu_inputs(T, seed=7200 + T)]
+        weights = hp.gpu_shard(0, 32)
+        cases[T] = (dev, weights, _fresh(pkg, dev, weights, T))
+    torch.cuda.synchronize()
+    own = [torch.cuda.Stream() for _ in range(2)]
+    assert all(s.stream_id & 1 for s in own) and torch.cuda.default_stream().stream_id == 0
+    foreign = torch.cuda.ExternalStream(own[1].cuda_stream)
+    assert foreign.stream_id != 0 and foreign.stream_id & 1 == 0
+    wrong = []
+
+    def work(streams):
+        outs = []
+        for k in range(30):
+            for T, (dev, weights, want) in cases.items():
+                with torch.cuda.stream(streams[k % len(streams)]):
+                    out = torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+                    pkg.run(*dev, *weights, 0, RSF, out)
+                outs.append((out, want))
+        torch.cuda.synchronize()
+        wrong.extend(not torch.equal(out.view(torch.int16), want) for out, want in outs)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in ([own[0], torch.cuda.default_stream()], [foreign])]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(wrong) == 180 and not any(wrong)
