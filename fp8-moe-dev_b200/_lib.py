@@ -37,7 +37,7 @@ EXPORTS = [
     "moe_fp8_b200_exchange_regions", "moe_fp8_b200_copy_rows_h2d",
     "moe_fp8_b200_invalidate_weights", "moe_fp8_b200_copy_device", "moe_fp8_b200_signal_peers",
     "moe_fp8_b200_wait_peers", "moe_fp8_b200_create_shaped", "moe_fp8_b200_workspace_bytes_shaped",
-    "moe_fp8_b200_get_shape",
+    "moe_fp8_b200_get_shape", "moe_fp8_b200_host_path",
 ]
 NOALLOC_MAX_TOKENS = 4096
 
@@ -106,6 +106,8 @@ def load() -> C.CDLL:
         fn = getattr(lib, name)
         fn.restype = C.c_int
         fn.argtypes = [H, C.POINTER(Args), C.c_void_p]
+    lib.moe_fp8_b200_host_path.restype = C.c_int
+    lib.moe_fp8_b200_host_path.argtypes = [H]
     lib.moe_fp8_b200_exchange_bytes.restype = C.c_size_t
     lib.moe_fp8_b200_exchange_bytes.argtypes = [C.c_int, C.c_int]
     lib.moe_fp8_b200_copy_device.restype = C.c_int

@@ -180,6 +180,7 @@ struct moe_fp8_b200_ctx {
     // staging for run_host (allocated on its first use)
     uint8_t* stage = nullptr;
     size_t stage_bytes = 0;
+    int host_path = 0;        // what the latest run_host did (moe_fp8_b200_host_path)
     // run_host with pinned buffers: the rows without a local expert are written on a stream of their own
     cudaStream_t side = nullptr;
     cudaEvent_t side_begin = nullptr, side_done = nullptr;
@@ -402,7 +403,8 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
 }
 
 // The device's address of host memory that kernels can reach: [p, p + bytes) lies inside one pinned, mapped
-// allocation.  Anything else (pageable, managed, device memory, a range that leaves its allocation) is not taken.
+// allocation, on a 4-byte boundary (the fetch kernel reads 32-bit words, where a copy takes any address).  Anything
+// else (pageable, managed, device memory, a range that leaves its allocation) is not taken.
 bool pinned_range(const void* p, size_t bytes, const void*& dev)
 {
     cudaPointerAttributes at;
@@ -422,7 +424,7 @@ bool pinned_range(const void* p, size_t bytes, const void*& dev)
     if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
         get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS)
         return false;
-    if (d < start || bytes > size || d - start > size - bytes) return false;
+    if (d < start || bytes > size || d - start > size - bytes || (d & 3u)) return false;
     dev = at.devicePointer;
     return true;
 }
@@ -924,6 +926,7 @@ int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, 
                         pinned_range(args->hidden_states_scale, n_scale, p_scale) && pinned_range(args->output, n_out, p_out) &&
                         !overlap(p_out, n_out, p_logits, n_logits) && !overlap(p_out, n_out, p_hidden, n_hidden) &&
                         !overlap(p_out, n_out, p_scale, n_scale);
+    h->host_path = direct ? 2 : 1;
     if (direct) {
         const bool zero_aside = h->num_local_experts <= kZeroAsideExperts && T >= kZeroAsideTokens;
         if (zero_aside && !h->side_done) {
@@ -962,6 +965,8 @@ int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, 
     if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "device-to-host copy: %s", cudaGetErrorString(e));
     return MOE_FP8_B200_OK;
 }
+
+int moe_fp8_b200_host_path(moe_fp8_b200_handle h) { return h ? h->host_path : MOE_FP8_B200_ERR_INVALID_ARGUMENT; }
 
 int moe_fp8_b200_run_host_async(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, void* stream_v, int64_t* ticket)
 {

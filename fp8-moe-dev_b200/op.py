@@ -337,6 +337,12 @@ class MoeLayer:
             self._raise(rc)
         return output
 
+    HOST_PATHS = (None, "copies", "in place")
+
+    def host_path(self):
+        """How the latest run_host moved its tensors."""
+        return self.HOST_PATHS[self._lib.moe_fp8_b200_host_path(self._h)]
+
     def run_host_async(self, routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights,
                        gemm1_weights_scale, gemm2_weights, gemm2_weights_scale, local_expert_offset,
                        routed_scaling_factor, output, stream: Optional[int] = None) -> int:

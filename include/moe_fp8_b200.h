@@ -206,9 +206,12 @@ MOE_FP8_B200_API int moe_fp8_b200_run(moe_fp8_b200_handle h, const moe_fp8_b200_
 /* Same layer with HOST pointers for the per-call tensors (routing_logits,
  * hidden_states, hidden_states_scale, output); routing_bias and the weights stay device
  * pointers.  Copies in, runs, copies out and synchronises `stream`; where all four lie in pinned, mapped
- * allocations the kernels read and write them in place instead of copying.  This is the
- * end-to-end form a host-resident caller of the reference operator sees. */
+ * allocations (logits and scales on a 4-byte boundary) the kernels read and write them in place instead of
+ * copying.  This is the end-to-end form a host-resident caller of the reference operator sees. */
 MOE_FP8_B200_API int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, void* stream);
+/* Diagnostics: how the handle's latest moe_fp8_b200_run_host moved its tensors: 0 no such call yet, 1 copies, 2 in
+ * place. */
+MOE_FP8_B200_API int moe_fp8_b200_host_path(moe_fp8_b200_handle h);
 
 /* Pipelined form of moe_fp8_b200_run_host for a caller that feeds batch after batch from host
  * memory: the call enqueues copy-in, the layer and copy-out on three streams and returns a

@@ -1,5 +1,7 @@
 """run_host with pinned buffers, which the kernels reach in place, against the copying form (pageable buffers)
 and the device-resident call: the same bits in every row, those of tokens without a local expert among them."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -62,5 +64,79 @@ def test_output_over_an_input_is_taken(pkg):
         out = block.view(torch.bfloat16).view(T, 7168)
         layer.run_host(inputs[0].pin_memory(), inputs[1].cuda(), hid, inputs[3].pin_memory(), *weights, 0, RSF, out)
         assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+    finally:
+        layer.close()
+
+
+@pytest.mark.parametrize("T,which", [(4, "logits"), (40, "logits"), (40, "scale"), (300, "both")])
+def test_floats_off_their_boundary_are_copied(pkg, T, which):
+    """Pinned logits or scales at any byte address: taken as before, through the copies, which take any address."""
+    layer = pkg.MoeLayer(512, 32, 0)
+    try:
+        inputs = hp.cpu_inputs(T, seed=80 + T)
+        weights = hp.gpu_shard(0, 32)
+        want = hp.run_layer(layer, inputs, weights, 0).cpu()
+        bias, out = inputs[1].cuda(), torch.empty(T, 7168, dtype=torch.bfloat16).pin_memory()
+        for off in (1, 2, 3, 4, 6):
+            blocks = []
+            for x, moved in ((inputs[0], which != "scale"), (inputs[3], which != "logits")):
+                at = off if moved else 0
+                block = torch.zeros(x.numel() * 4 + 16, dtype=torch.uint8).pin_memory()
+                block[at:at + x.numel() * 4].copy_(x.reshape(-1).view(torch.uint8))
+                blocks.append((block, block.data_ptr() + at))
+            hidden = inputs[2].pin_memory()
+            a = pkg._lib.Args(blocks[0][1], bias.data_ptr(), hidden.data_ptr(), blocks[1][1], *(w.data_ptr() for w in weights),
+                              0, RSF, out.data_ptr(), T)
+            out.fill_(7.0)
+            rc = layer._lib.moe_fp8_b200_run_host(layer._h, C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+            assert rc == 0, layer._lib.moe_fp8_b200_last_error(layer._h)
+            assert layer.host_path() == ("in place" if off == 4 else "copies")
+            assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+        layer.check()
+    finally:
+        layer.close()
+
+
+# both sides of the rules: 128 experts copy above 1024 tokens; 256 experts never; empty rows leave aside from 256
+# tokens on up to 64 experts
+@pytest.mark.parametrize("T,E,path", [(8, 32, "in place"), (256, 64, "in place"), (1024, 128, "in place"), (1025, 128, "copies"),
+                                      (1025, 256, "in place"), (2048, 32, "in place")])
+def test_which_path_a_pinned_call_takes(pkg, T, E, path):
+    """... and that new contents of the same pinned buffers are seen."""
+    layer = pkg.MoeLayer(T, E, 0)
+    try:
+        weights = hp.gpu_shard(0, E)
+        src = [None if i == 1 else x.pin_memory() for i, x in enumerate(hp.cpu_inputs(T, seed=90))]
+        out = torch.empty(T, 7168, dtype=torch.bfloat16).pin_memory()
+        assert layer.host_path() is None
+        for seed in (91, 92):
+            inputs = hp.cpu_inputs(T, seed=seed)
+            want = hp.run_layer(layer, inputs, weights, 0).cpu()
+            for i in (0, 2, 3):
+                src[i].copy_(inputs[i])
+            layer.run_host(src[0], inputs[1].cuda(), src[2], src[3], *weights, 0, RSF, out)
+            assert layer.host_path() == path
+            assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+        layer.run_host(inputs[0], inputs[1].cuda(), inputs[2], inputs[3], *weights, 0, RSF, torch.empty_like(want))
+        assert layer.host_path() == "copies"      # pageable
+    finally:
+        layer.close()
+
+
+@pytest.mark.parametrize("T", [5, 255, 256, 700])
+def test_no_token_has_an_expert_here(pkg, T):
+    """Every selected expert lies outside the shard: no tile, no row; the output is zeros, written aside from 256
+    tokens on."""
+    layer = pkg.MoeLayer(700, 32, 0)
+    try:
+        logits, bias, hid, scale = hp.cpu_inputs(T, seed=95)
+        logits = logits - 8.0
+        logits[:, 64:72] += 16.0
+        weights = hp.gpu_shard(0, 32)
+        out = torch.full((T, 7168), 7.0, dtype=torch.bfloat16).pin_memory()
+        layer.run_host(logits.pin_memory(), (bias * 0).cuda(), hid.pin_memory(), scale.pin_memory(), *weights, 0, RSF, out)
+        assert layer.host_path() == "in place" and torch.count_nonzero(out) == 0
+        assert layer.read("expert_count", 32).sum() == 0
+        layer.check()
     finally:
         layer.close()
