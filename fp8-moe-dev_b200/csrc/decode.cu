@@ -319,6 +319,9 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
                 sh->r_sel[t][rank] = r_s[t * kNumExperts + ge];
             }
         }
+        // The scratch lies in half 0's first ring slots, which TMA writes next: ordinary accesses and the async
+        // proxy's to the same bytes want this fence, by every thread that made them, in front of the barrier.
+        fence_proxy_async_smem();
     } else if (warp < T) {
         // more tokens than that: one warp per token runs the staged chain's routine, the tokens in parallel
         int idx[kTopK];

@@ -173,3 +173,24 @@ def test_decode_routing_equals_chain_routing_on_many_batches_and_ties(pkg, layer
         assert np.array_equal(td[0], tc[0]), f"trial {trial}: expert picks differ"
         assert np.array_equal(td[1], tc[1]), f"trial {trial}: weights differ"
         assert np.array_equal(td[2], tc[2]) and td[3] == tc[3] and np.array_equal(td[4], tc[4])
+
+
+@pytest.mark.parametrize("T", [1, 2, 3])
+def test_cooperative_routing_under_the_first_weights(layers, T):
+    """Up to three tokens are routed in shared memory that the first weight steps then fill: the tables are the
+    chain's and the rows too, call after call behind one another."""
+    dec, chain = layers
+    weights = hp.gpu_shard(32, 32)
+    cases = [[x.cuda() for x in hp.cpu_inputs(T, seed=1500 + 40 * T + k)] for k in range(24)]
+    outs = [torch.empty(T, H, dtype=torch.bfloat16, device="cuda") for _ in cases]
+    dec.invalidate_weights()
+    for inputs, out in zip(cases, outs):
+        dec.run(*inputs, *weights, 32, RSF, out)
+    dec.check()
+    for inputs, out in zip(cases, outs):
+        want = hp.run_layer(chain, inputs, weights, 32)
+        alone = hp.run_layer(dec, inputs, weights, 32)
+        tab_dec, tab_chain = _tables(dec, T), _tables(chain, T)
+        assert all(np.array_equal(tab_dec[i], tab_chain[i]) for i in (0, 1, 2, 4)) and tab_dec[3] == tab_chain[3]
+        assert torch.equal(out.view(torch.int16), alone.view(torch.int16))
+        assert hp.error_stats(out.float().cpu().numpy(), want.float().cpu().numpy())["rel_l2"] < 5e-3
