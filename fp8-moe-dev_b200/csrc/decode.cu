@@ -90,6 +90,7 @@ struct DecodeShared {
     int r_idx[kDecodeMaxTokens][kTopK];
     float r_sel[kDecodeMaxTokens][kTopK];
     float hid_scale[kDecodeMaxTokens][kHiddenBlocks];      // [token][kb]
+    int stop_at[2];                                        // per half: ring position (2 slot + parity) no step will fill, or -1
     alignas(16) int4 step_desc[2][kRingFew];               // {unit, step, next unit or -1, -}; unit -1: no more
     alignas(8) uint64_t full_bar[2][kRingFew];
     alignas(8) uint64_t empty_bar[2][kRingFew];
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
     pdl_launch_dependents();
     if (tid == 0) {
         sh->abort = 0;
+        sh->stop_at[0] = sh->stop_at[1] = -1;
         prefetch_tmap(&tmap_w1);
         prefetch_tmap(&tmap_w2);
         mbar_init(smem_u32(&sh->hid_bar), 1);
@@ -488,6 +490,8 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
             sh->step_desc[half][slot] = make_int4(-1, 0, -1, 0);
             mbar_arrive(smem_u32(&full_bar[slot]));
         } else {
+            // This is where the half stops: the consumers take every step issued so far and find the position here.
+            *(volatile int*)&sh->stop_at[half] = 2 * slot + (int)(phase ^ 1u);
             // leave only after the copies in flight have landed (bounded)
             for (int g = issued > ring ? issued - ring : 0; g < issued; ++g) {
                 const uint32_t bar = smem_u32(&full_bar[g % ring]);
@@ -506,8 +510,23 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
         if (lane == 0) mbar_arrive(smem_u32(&empty_bar[slot]));
         if (++slot == ring) { slot = 0; phase ^= 1u; }
     };
-    // waits for the next step; false: this half gives up
-    auto arrived = [&]() -> bool { return mbar_wait(smem_u32(&full_bar[slot]), phase, abort_flag); };
+    // Waits for the next step; false: the half ends here.  The eight warps meet once per unit at a named barrier,
+    // which has no limit of its own, so all of them must end at the same step.  Their producer alone decides which:
+    // it issues a step or, when one of its waits runs out or the CTA's abort flag is up, names the ring position where
+    // it stopped; a step that was issued arrives.  (No other position has that slot and parity: the producer is at
+    // most one ring ahead.)  The abort flag itself is not looked at here, since one warp might find its step arrived
+    // and another one the flag.  The limit behind it is for a copy that never lands: longer than any wait of the
+    // producer, and then no warp of the half gets past that step.
+    const volatile int* stop_at = &sh->stop_at[half];
+    auto arrived = [&]() -> bool {
+        const uint32_t bar = smem_u32(&full_bar[slot]);
+        if (mbar_try_wait(bar, phase)) return true;
+        const uint64_t t0 = global_timer_ns();
+        for (uint32_t it = 1;; ++it) {
+            if (mbar_try_wait(bar, phase)) return true;
+            if ((it & 0xffu) == 0u && (*stop_at == 2 * slot + (int)phase || global_timer_ns() - t0 > 4 * kWaitLimitNs)) return false;
+        }
+    };
     // the first step of the next unit and what the producer wrote about it ({-1, ...} once there is no more work)
     int4 d = make_int4(-1, 0, -1, 0);
     auto next_unit = [&]() {
@@ -533,8 +552,9 @@ __global__ void __launch_bounds__(kDecThreads, 1) decode_layer_kernel(
         }
         return v;
     };
-    // the hidden rows must have landed before the first MMA
-    if (!mbar_wait(smem_u32(&sh->hid_bar), 0u, abort_flag)) ok = false;
+    // the hidden rows must have landed before the first MMA (a wait that fails sets the abort flag and is reported at
+    // the end: a warp does not leave its half, see arrived)
+    mbar_wait(smem_u32(&sh->hid_bar), 0u, abort_flag);
 
     float sc_next = 0.0f;
     int loaded_for = -1;   // unit that sc_next belongs to
