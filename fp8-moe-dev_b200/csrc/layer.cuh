@@ -27,6 +27,8 @@ constexpr int kMaxLocalExperts = 256;
 // (one per work unit).
 constexpr int kSplitKSlots = 320;
 
+constexpr int kZeroCtas = 3;         // CTAs of zero_rows_kernel, and SMs that the GEMMs leave free beside it
+
 // What the dispatch step does with a token's experts that fall into one 32-expert
 // shard.  The fields restate, as data, the branch structure of the reference's
 // routing kernel (kernel/moe_fp8.cu:457-607) after its compile-time knobs
@@ -72,13 +74,12 @@ struct Control {
     int status;                          // 0 ok; otherwise the first error a kernel recorded
     int status_detail;
     int blocks_done;                     // routing CTAs finished (ticket for the last-CTA scan)
-    int permute_done;                    // permute CTAs finished, where zero_rows_kernel asks (zeroed by the routing kernel's scan)
     int expert_rows[kMaxLocalExperts];   // copy of the counters of the last call (diagnostics)
     int splitk_ticket[kSplitKSlots];     // per-tile arrival counters of the split-K reduction (self-clearing)
     int unit_ticket[2];                  // next work unit of the fused expert GEMMs (zeroed by the routing kernel's scan)
     int push_done;                       // combine-and-push CTAs finished (ticket, self-clearing)
     unsigned dec_ticket;                 // next run of work units of the decode kernel (cleared by its combine)
-    int pad2[2];
+    int pad2[3];
     unsigned long long dec_time[16];     // phase timestamps (ns) of CTA 0 in the last decode-kernel run
     // Timestamps (ns, %globaltimer) of the last fused combine + reduce-scatter on this rank:
     // [0] first CTA of the push starts, [1] last CTA of the push done (flags published), [2] first CTA of the

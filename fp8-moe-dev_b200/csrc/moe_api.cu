@@ -17,7 +17,7 @@
 namespace moe {
 cudaError_t launch_route_dispatch(const float*, const void*, const Workspace&, int, int, int, float,
                                   const DispatchPolicy&, int, cudaStream_t);
-cudaError_t launch_permute(const void*, const float*, const Workspace&, int, int, cudaStream_t);
+cudaError_t launch_permute(const void*, const float*, const Workspace&, int, cudaStream_t);
 cudaError_t launch_combine(const Workspace&, void*, int, int, int, cudaStream_t);
 cudaError_t launch_zero_rows(const Workspace&, void*, int, cudaStream_t);
 cudaError_t launch_fetch_inputs(const FetchList&, int, cudaStream_t);
@@ -348,12 +348,6 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
         e = launch_route_dispatch(a.routing_logits, a.routing_bias, h->ws, T, (int)a.local_expert_offset, E,
                                   (float)a.routed_scaling_factor, pol, /*do_scan=*/1, stream);
     mark(1);
-    if (zero_aside) {
-        if (e == cudaSuccess) e = cudaEventRecord(h->side_begin, stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->side_begin, 0);
-        if (e == cudaSuccess) e = launch_zero_rows(h->ws, a.output, T, h->side);
-        if (e == cudaSuccess) e = cudaEventRecord(h->side_done, h->side);
-    }
     mark(2);
     const int stop = h->opt_stop_after > 0 ? h->opt_stop_after : 99;
     // decode-sized batches may leave most SMs without a tile: there the split-K instantiation
@@ -361,13 +355,19 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
     const int split_k = (T <= 4 && ref_geo) ? 1 : 0;   // 4 = kSplitKMaxRows of the GEMM kernel
     // at most 64 tokens (an expert then has at most 64 rows): 64-row activation boxes and a fourth operand stage
     const int small_a = (h->opt_small_batch_ring && T > 4 && T <= 64 && ref_geo) ? 1 : 0;
-    if (e == cudaSuccess && stop >= 2) e = launch_permute(a.hidden_states, a.hidden_states_scale, h->ws, T, zero_aside ? 1 : 0, stream);
+    if (e == cudaSuccess && stop >= 2) e = launch_permute(a.hidden_states, a.hidden_states_scale, h->ws, T, stream);
+    if (zero_aside) {
+        if (e == cudaSuccess) e = cudaEventRecord(h->side_begin, stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->side_begin, 0);
+        if (e == cudaSuccess) e = launch_zero_rows(h->ws, a.output, T, h->side);
+        if (e == cudaSuccess) e = cudaEventRecord(h->side_done, h->side);
+    }
     mark(3);
     const GemmMaps maps = {small_a ? h->tmap_a1_small : h->tmap_a1, tiled ? h->tmap_w1_tiled : h->tmap_w1,
                            small_a ? h->tmap_a2_small : h->tmap_a2, tiled ? h->tmap_w2_tiled : h->tmap_w2, h->tmap_y};
-    // one persistent CTA per SM (a CTA takes all of an SM's registers: one SM is left to zero_rows_kernel where that
+    // one persistent CTA per SM (a CTA takes all of an SM's registers: some SMs are left to zero_rows_kernel where that
     // runs); CTAs without work leave at once
-    const int gemm_ctas = zero_aside && h->num_sms > 1 ? h->num_sms - 1 : h->num_sms;
+    const int gemm_ctas = zero_aside && h->num_sms > kZeroCtas ? h->num_sms - kZeroCtas : h->num_sms;
     auto gemms = [&](int phases) {
         return launch_expert_gemms(maps, gemm_ws, scale1, scale2, h->opt_exact_silu, phases, gemm_ctas, small_a, stream);
     };

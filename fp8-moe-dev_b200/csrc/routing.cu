@@ -54,7 +54,6 @@ __device__ __forceinline__ void scan_tiles_block(const Workspace& ws, int num_lo
         ws.expert_offset[num_local_experts] = total * kTileM;
         ws.num_tiles[0] = total;
         ws.ctrl->blocks_done = 0;
-        ws.ctrl->permute_done = 0;
         ws.ctrl->unit_ticket[0] = ws.ctrl->unit_ticket[1] = 0;
         // the status word is sticky: the first failure stays until the host has read it
         if (overflow && atomicCAS(&ws.ctrl->status, kStatusOk, kStatusRowOverflow) == kStatusOk)
@@ -208,13 +207,8 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_dispatch_kernel(
 // ---------------------------------------------------------------------------------------
 constexpr int kPermuteWarps = 4;
 
-// `count_done`: zero_rows_kernel waits for the permute's reads of host memory; a warp that is done with them says so.
-__device__ __forceinline__ void count_permuted(const Workspace& ws, int lane, int count_done) {
-    if (count_done && lane == 0) atomicAdd(&ws.ctrl->permute_done, 1);
-}
-
 __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_kernel(
-    const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, Workspace ws, int T, int count_done)
+    const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, Workspace ws, int T)
 {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kPermuteWarps + (threadIdx.x >> 5);
@@ -230,7 +224,7 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_kernel(
         }
         ws.pair_row[(size_t)t * kTopK + lane] = r;
     }
-    if (n_pairs == 0) { count_permuted(ws, lane, count_done); return; }
+    if (n_pairs == 0) return;
 
     constexpr int kVec = kHidden / 16 / 32;  // 14 uint4 per lane
     uint4 v[kVec];
@@ -252,12 +246,11 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_kernel(
         if (lane + 32 < kHiddenBlocks) ws.sfa1[(size_t)(lane + 32) * ws.m_cap + row] = sc1;
         if (lane == 0) ws.row_token[row] = t;
     }
-    count_permuted(ws, lane, count_done);
 }
 
 // The same movement for a run-time row length (Workspace::geo.hidden, a multiple of 256 bytes, at most 8192).
 __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_generic_kernel(
-    const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, Workspace ws, int T, int count_done)
+    const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale, Workspace ws, int T)
 {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kPermuteWarps + (threadIdx.x >> 5);
@@ -273,7 +266,7 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_generic_kerne
         }
         ws.pair_row[(size_t)t * kTopK + lane] = r;
     }
-    if (n_pairs == 0) { count_permuted(ws, lane, count_done); return; }
+    if (n_pairs == 0) return;
     const int H = ws.geo.hidden;
     const int vecs = H / 16, blocks = H / kBlock;   // <= 512 uint4, <= 64 scales
     const uint4* src = reinterpret_cast<const uint4*>(hidden + (size_t)t * H);
@@ -295,7 +288,6 @@ __global__ void __launch_bounds__(kPermuteWarps * 32) permute_rows_generic_kerne
         if (lane + 32 < blocks) ws.sfa1[(size_t)(lane + 32) * ws.m_cap + row] = sc1;
         if (lane == 0) ws.row_token[row] = t;
     }
-    count_permuted(ws, lane, count_done);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -474,24 +466,20 @@ __global__ void __launch_bounds__(kFetchThreads) fetch_inputs_kernel(const __gri
     }
 }
 
-// Output rows of the tokens that have no expert here (most of them where a GPU holds one shard of eight): known as
-// soon as routing is done, written to the host while the experts' GEMMs run, for which these leave one SM free.
-// Bound by PCIe, which few CTAs of plain stores fill (52 GB/s from 8 CTAs as from 296; cudaMemcpyAsync 56.7); four
-// of 512 threads fit on that one SM.  A warp per row.
-constexpr int kZeroCtas = 4, kZeroThreads = 512;
+// Output rows of the tokens that have no expert here (most of them where a GPU holds one shard of eight), written to
+// the host while the experts' GEMMs run, for which these leave an SM free per CTA.  On a stream of its own behind the
+// permute: not earlier, because the permute's read requests would queue behind these writes on their way out (host
+// call on 32 experts, beside the permute / behind it: T=512 369 / 337 us, T=1024 520 / 474), and by then the GEMMs'
+// CTAs hold all other SMs (the combine's, which would take the free ones, start behind the GEMMs in these calls).
+// Bound by PCIe, which few CTAs of plain stores fill if they do not share an SM (32 experts, T=1024 / 2048 / 4096, us:
+// four CTAs on one SM 440 / 810 / 1575, two on two 429 / 765 / 1491, three on three 423 / 765 / 1489, four on four
+// 425 / 764 / 1490).  A warp per row.
+constexpr int kZeroThreads = 512;
 __global__ void __launch_bounds__(kZeroThreads) zero_rows_kernel(Workspace ws, uint8_t* __restrict__ out, int T)
 {
     const int lane = threadIdx.x & 31, warps = kZeroCtas * (kZeroThreads / 32);
     const bool none = ws.num_tiles[0] == 0;
     const int vecs = ws.geo.hidden * 2 / 16;
-    // Not before the permute has read its rows: its read requests would queue behind these writes on their way out
-    // (host call on 32 experts: T=512 369 us without this wait, 337 with it; T=1024 520 / 474).  Resident already,
-    // because the combine's CTAs would take the free SM.  The wait is a courtesy, nothing depends on its outcome.
-    if (threadIdx.x == 0) {
-        const uint64_t t0 = global_timer_ns();
-        while (*reinterpret_cast<volatile int*>(&ws.ctrl->permute_done) < T && global_timer_ns() - t0 < 5000000ull) __nanosleep(500);
-    }
-    __syncthreads();
     for (int t = blockIdx.x * (kZeroThreads / 32) + (threadIdx.x >> 5); t < T; t += warps) {
         if (!none && ws.pair_count[t] != 0) continue;
         uint4* row = reinterpret_cast<uint4*>(out) + (size_t)t * vecs;
@@ -500,11 +488,11 @@ __global__ void __launch_bounds__(kZeroThreads) zero_rows_kernel(Workspace ws, u
 }
 
 // ---------------------------------------------------------------------------------------
-// Launchers (called by the C-ABI layer).  All launches carry the programmatic stream
-// serialization attribute (see ptx.cuh).
+// Launchers (called by the C-ABI layer).  All launches but two carry the programmatic stream
+// serialization attribute (see ptx.cuh): zero_rows_kernel, and the combine beside it.
 // ---------------------------------------------------------------------------------------
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+static cudaError_t launch_one(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args... args)
 {
     cudaLaunchConfig_t cfg = {};
@@ -516,8 +504,13 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)
+{
+    return launch_one(true, kernel, grid, block, smem, stream, args...);
 }
 
 cudaError_t launch_route_dispatch(const float* logits, const void* bias, const Workspace& ws, int T,
@@ -534,25 +527,24 @@ cudaError_t launch_route_dispatch(const float* logits, const void* bias, const W
                       do_scan);
 }
 
-cudaError_t launch_permute(const void* hidden, const float* hidden_scale, const Workspace& ws, int T, int count_done,
-                           cudaStream_t stream)
+cudaError_t launch_permute(const void* hidden, const float* hidden_scale, const Workspace& ws, int T, cudaStream_t stream)
 {
     const int grid = (T + kPermuteWarps - 1) / kPermuteWarps;
     if (!ws.geo.is_reference())
         return launch_pdl(permute_rows_generic_kernel, dim3(grid), dim3(kPermuteWarps * 32), 0, stream,
-                          static_cast<const uint8_t*>(hidden), hidden_scale, ws, T, count_done);
+                          static_cast<const uint8_t*>(hidden), hidden_scale, ws, T);
     return launch_pdl(permute_rows_kernel, dim3(grid), dim3(kPermuteWarps * 32), 0, stream,
-                      static_cast<const uint8_t*>(hidden), hidden_scale, ws, T, count_done);
+                      static_cast<const uint8_t*>(hidden), hidden_scale, ws, T);
 }
 
 cudaError_t launch_combine(const Workspace& ws, void* out, int T, int skip_empty, int from_views, cudaStream_t stream)
 {
     __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
     if (!ws.geo.is_reference())
-        return launch_pdl(from_views ? combine_generic_kernel<true> : combine_generic_kernel<false>, dim3(T), dim3(256), 0, stream,
-                          ws, o, T, skip_empty);
-    return launch_pdl(from_views ? combine_kernel<true> : combine_kernel<false>, dim3(T), dim3(kCombineThreads), 0, stream, ws, o,
-                      T, skip_empty);
+        return launch_one(!skip_empty, from_views ? combine_generic_kernel<true> : combine_generic_kernel<false>, dim3(T),
+                          dim3(256), 0, stream, ws, o, T, skip_empty);
+    return launch_one(!skip_empty, from_views ? combine_kernel<true> : combine_kernel<false>, dim3(T), dim3(kCombineThreads), 0,
+                      stream, ws, o, T, skip_empty);
 }
 
 cudaError_t launch_zero_rows(const Workspace& ws, void* out, int T, cudaStream_t stream)
