@@ -1,7 +1,5 @@
 """The kernels that draw their work: the expert GEMMs at the edges of their 128-row tiles, as one launch and cut
 between the two GEMMs, and the decode kernel where its rows are handed from phase to phase."""
-import time
-
 import numpy as np
 import pytest
 import torch
@@ -84,34 +82,3 @@ def test_decode_rows_between_the_phases(pkg, rows_a, rows_b, T):
     finally:
         dec.close()
         chain.close()
-
-
-@pytest.mark.parametrize("rows_a,rows_b,T", [(1, 0, 1), (2, 1, 3), (5, 3, 8)])
-def test_decode_wait_that_runs_out(pkg, rows_a, rows_b, T):
-    """Rows that never come: the work counter is set, from the host, past the runs of phase 1, so every worker draws
-    phase 2 and waits for activations that nobody makes.  The waits run out after their second, both halves of every
-    CTA leave, the launch completes, check() reports it and the next call is right again."""
-    layer = pkg.MoeLayer(16, 32, 0)
-    try:
-        inputs = _inputs(rows_a, rows_b, T, 950 + T)
-        weights = hp.gpu_shard(OFFSET, 32)
-        want = hp.run_layer(layer, inputs, weights, OFFSET).clone()
-        units = 256 * ((rows_a > 0) + (rows_b > 0))
-        workers = 2 * torch.cuda.get_device_properties(0).multi_processor_count
-        runs = units // 8 * 7 if units >= 2 * workers else 0
-        rest = units - runs
-        each = max(1, rest // (4 * workers))
-        layer.inject_device_status(0, (workers if runs else 0) + -(-rest // each))
-        dev = [x.cuda() for x in inputs]
-        out = torch.zeros(T, hp.H, dtype=torch.bfloat16, device="cuda")
-        torch.cuda.synchronize()
-        t0 = time.perf_counter()
-        layer.run(*dev, *weights, OFFSET, RSF, out)
-        with pytest.raises(pkg.MoeError) as ei:
-            layer.check()
-        dt = time.perf_counter() - t0
-        assert ei.value.code == -4 and "105" in str(ei.value), str(ei.value)
-        assert 0.9 < dt < 3.0, dt
-        assert torch.equal(hp.run_layer(layer, inputs, weights, OFFSET).view(torch.int16), want.view(torch.int16))
-    finally:
-        layer.close()
