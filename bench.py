@@ -309,9 +309,9 @@ def small_config_latencies(pkg, weights, bias_dev, reference_mod=None):
         wall = (time.perf_counter() - t0) / 100 * 1e6
         timeline = None
         if T <= 8:
-            # the decode kernel's own phase clock (CTA 0, ns), median over 20 eager runs
+            # the decode kernel's own phase clock (CTA 0, then its combine kernel; ns), median over 20 eager runs
             import numpy as np
-            names = ("tables", "phase1_gemm1_swiglu", "barrier1_wait", "phase2_requant_gemm2", "barrier2_wait", "combine")
+            names = ("tables", "phase1_gemm1_swiglu", "first_rows_of_phase2", "phase2_gemm2", "until_combine", "combine")
             acc = []
             for _ in range(20):
                 run()
@@ -493,7 +493,8 @@ def run_ours(args, rank, world, local):
     # Stage times come from a pass of their own: while they are recorded the two GEMMs run as two launches of
     # the kernel that otherwise does both.
     layer.set_stage_timing(True)
-    time_steps(step, min(args.steps, 30), args.warmup, world)
+    with ClockSampler(local) as stage_clk:
+        time_steps(step, min(args.steps, 30), args.warmup, world)
     stages, timed_runs = layer.stage_times()
     layer.set_stage_timing(False)
     layer.check()
@@ -656,6 +657,8 @@ def run_ours(args, rank, world, local):
                                   f"nominal dense fp8 {FP8_NOMINAL_TFLOPS:.0f}",
                      "frac_of_nominal": round(achieved / FP8_NOMINAL_TFLOPS, 4),
                      "flops_per_launch": g1_flops, "avg_launch_ms": round(g1_ms, 4), "timed_launches": timed_runs,
+                     "timed_in": "a pass of its own behind the timed steps, GEMM1 and GEMM2 as two launches",
+                     "clocks": stage_clk.summary(),
                      "traffic": (NCU_GEMM1_DRAM_BYTES_32_EXPERTS_T12288 * E / 32) if T >= 8192 else None,
                      "traffic_note": "SCALED, not measured at this size: ncu dram bytes of GEMM1 at T=12288 on one "
                                      "32-expert shard (928 MB, weights 96 % of it and read once) x experts/32"},

@@ -26,7 +26,7 @@
 //   * the weighted combine is a kernel of its own (decode_combine_kernel): it is resident before this one ends,
 //     so its start costs no more than a grid barrier would, and meanwhile the CTAs of the next
 //     layer's decode kernel, which need this one's shared memory, can move in.
-// Every wait is bounded.
+// Every wait on memory or an mbarrier is bounded; the named barrier of a half is met by all of its warps or none.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -75,7 +75,7 @@ static_assert(kDecodeMaxTokens * kHidStride % 128 == 0 && kFewTokens * kHidStrid
 static_assert(2 * kDecodeMaxTokens * kNumExperts * 4 <= 2 * kRing * kStepBytes, "routing scratch fits the idle rings");
 
 struct DecodeShared {
-    int n_rows, abort;
+    int abort;
     int pair_count[kDecodeMaxTokens];
     int pair_le[kDecMaxActive];                            // [token][pair] local expert, -1 past the token's pairs
     int pair_first[kDecMaxActive];                         // entry of that expert's first use

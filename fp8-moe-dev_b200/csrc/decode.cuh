@@ -17,9 +17,7 @@ struct DecodeArgs {
     const __nv_bfloat16* bias;      // [256]
     const uint8_t* hidden;          // [T, 7168] e4m3
     const float* hscale;            // [56, T]
-    const uint8_t* w1;              // [E, 4096, 7168] e4m3
-    const float* s1;                // [E, 32, 56]
-    const uint8_t* w2;              // [E, 7168, 2048] e4m3
+    const float* s1;                // [E, 32, 56] (the weights themselves come through the tensor maps)
     const float* s2;                // [E, 56, 16]
     __nv_bfloat16* out;             // [T, 7168]
     int T, local_expert_offset, num_local_experts;

@@ -504,16 +504,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
                 tmem_ld_32x32(t + c0, r0);
                 tmem_ld_32x32(t + c1, r1);
                 tmem_ld_wait2(r0, r1);
-                promote32<0, true>(acc, r0, s_lo);
+                promote32<0>(acc, r0, s_lo);
                 tmem_ld_32x32(t + c2, r0);
-                promote32<32, true>(acc, r1, s_lo);
+                promote32<32>(acc, r1, s_lo);
                 tmem_ld_32x32(t + c3, r1);
                 tmem_ld_wait2(r0, r1);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty[as]));
-                promote32<64, true>(acc, r0, s_hi);
-                promote32<96, true>(acc, r1, s_hi);
+                promote32<64>(acc, r0, s_hi);
+                promote32<96>(acc, r1, s_hi);
             }
             if (!ok) break;
 

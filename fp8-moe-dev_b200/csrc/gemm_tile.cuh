@@ -73,25 +73,19 @@ __device__ __forceinline__ void tmem_ld_wait2(uint32_t (&a)[32], uint32_t (&b)[3
                  : "memory");
 }
 
-// acc[OFF + j] += raw[j] * s for 32 accumulator columns.  PACKED uses the two-wide fp32 FMA of
-// sm_100: same IEEE result per element and the same FMA-pipe time, but half the issue slots.
+// acc[OFF + j] += raw[j] * s for 32 accumulator columns, by the two-wide fp32 FMA of sm_100: same IEEE result per element and the same FMA-pipe time, but half the issue slots.
 // That matters because the MMA-issuing thread shares its scheduler with two of these warps: long
 // bursts of scalar FMAs starve it (measured: 728 -> 592 cycles per K block in an isolated
 // two-stage pipeline when the promotion uses the packed form).
-template <int OFF, bool PACKED>
+template <int OFF>
 __device__ __forceinline__ void promote32(float (&acc)[128], const uint32_t (&r)[32], float s) {
-    if (PACKED) {
-        const float2 s2 = make_float2(s, s);
+    const float2 s2 = make_float2(s, s);
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-            const float2 d = __ffma2_rn(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), s2,
-                                        make_float2(acc[OFF + j], acc[OFF + j + 1]));
-            acc[OFF + j] = d.x;
-            acc[OFF + j + 1] = d.y;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) acc[OFF + j] = fmaf(__uint_as_float(r[j]), s, acc[OFF + j]);
+    for (int j = 0; j < 32; j += 2) {
+        const float2 d = __ffma2_rn(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), s2,
+                                    make_float2(acc[OFF + j], acc[OFF + j + 1]));
+        acc[OFF + j] = d.x;
+        acc[OFF + j + 1] = d.y;
     }
 }
 

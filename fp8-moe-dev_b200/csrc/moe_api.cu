@@ -46,15 +46,16 @@ namespace {
 constexpr int kVersion = (0 << 16) | 1;
 
 // run_host with pinned buffers, rows without a local expert written beside the GEMMs: pays where a GPU holds at most
-// a quarter of the experts (half to a quarter of the tokens have no row; with 128 experts 3 %, no difference) and
-// the batch has enough such rows (32 experts, written aside / by the combine: T=57 185 / 182 us, T=256 264 / 302,
-// T=2048 789 / 1009; 64 experts: T=128 378 / 372, T=256 460 / 468, T=2048 1300 / 1384).
+// a quarter of the experts (half to a quarter of the tokens have no row) and the batch has enough such rows (us,
+// written aside / by the combine: 32 experts T=57 181 / 182, T=128 207 / 219, T=256 244 / 283, T=2048 764 / 971; 64
+// experts T=128 355 / 353, T=256 426 / 440, T=2048 1192 / 1308; 128 experts T=1024 1243 / 1237).
 constexpr int kZeroAsideExperts = 64;
 constexpr int kZeroAsideTokens = 256;
 // Half of the experts: nearly every row moves (few zero rows to leave early) and the permute and combine under which
-// transfers can hide are half as long as with all of them, so that a copy engine's 8 % higher rate wins from about
-// a thousand tokens on (copies / in place: T=1024 1291 / 1263 us, T=4096 3057 / 3055, T=8192 5504 / 5565, T=16384
-// 10145 / 10315; all 256 experts: T=4096 4267 / 4230, T=12288 10062 / 10038).
+// transfers can hide are half as long as with all of them, so that a copy engine's 8 % higher rate wins, by little,
+// from about a thousand tokens on (us, copies / in place: T=256 752 / 741, T=512 938 / 924, T=1024 1240 / 1238, T=2048
+// 1812 / 1816, T=4096 3015 / 3034, T=8192 5582 / 5644, T=16384 10380 / 10400; all 256 experts: T=1024 1991 / 1982,
+// T=4096 4353 / 4316, T=12288 10293 / 10208).
 constexpr int kHalfOfExperts = 128;
 constexpr int kHalfInPlaceTokens = 1024;
 thread_local std::string g_create_error;
@@ -302,9 +303,7 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
         d.bias = static_cast<const __nv_bfloat16*>(a.routing_bias);
         d.hidden = static_cast<const uint8_t*>(a.hidden_states);
         d.hscale = a.hidden_states_scale;
-        d.w1 = static_cast<const uint8_t*>(a.gemm1_weights);
         d.s1 = a.gemm1_weights_scale;
-        d.w2 = static_cast<const uint8_t*>(a.gemm2_weights);
         d.s2 = a.gemm2_weights_scale;
         d.out = static_cast<__nv_bfloat16*>(a.output);
         d.T = T;
@@ -915,9 +914,9 @@ int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, 
     cudaError_t e = cudaSuccess;
     // Pinned buffers (and an output that shares no byte with an input): kernels read and write them in place, so that
     // rows without an expert here are never brought in, their zeros leave during the GEMMs, and no copy engine's
-    // start and end lies between the kernels.  Whole call, copies / in place: 32 experts T=16 149 / 135 us, T=256
-    // 339 / 264, T=2048 1130 / 789, T=4096 2050 / 1534; 256 experts, where every row moves and a copy engine is
-    // 8 % faster than a kernel's loads and stores, T=128 1178 / 1166, T=4096 4393 / 4359.
+    // start and end lies between the kernels.  Whole call, us, copies / in place: 32 experts T=16 158 / 145, T=256 334 /
+    // 244, T=2048 1118 / 764, T=4096 2034 / 1491; 64 experts T=2048 1349 / 1192; 256 experts, where every row moves and a
+    // copy engine is 8 % faster than a kernel's loads and stores, T=128 1194 / 1179 (128 and more: kHalfOfExperts).
     const bool decode_size = T <= kDecodeMaxTokens;
     const void *p_logits, *p_hidden, *p_scale, *p_out;
     const bool direct = h->opt_stop_after == 0 && (h->num_local_experts != kHalfOfExperts || T <= kHalfInPlaceTokens) &&
@@ -1149,13 +1148,13 @@ int moe_fp8_b200_check(moe_fp8_b200_handle h, void* stream)
     return MOE_FP8_B200_OK;
 }
 
-int moe_fp8_b200_inject_device_status(moe_fp8_b200_handle h, int status, unsigned stale_barrier_arrivals, void* stream)
+int moe_fp8_b200_inject_device_status(moe_fp8_b200_handle h, int status, unsigned stale_tickets, void* stream)
 {
     if (!h) return MOE_FP8_B200_ERR_INVALID_ARGUMENT;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaMemcpyAsync(&h->ws.ctrl->status, &status, sizeof(int), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&h->ws.ctrl->dec_ticket, &stale_barrier_arrivals, sizeof(unsigned), cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync(&h->ws.ctrl->dec_ticket, &stale_tickets, sizeof(unsigned), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "status injection: %s", cudaGetErrorString(e));
     return MOE_FP8_B200_OK;

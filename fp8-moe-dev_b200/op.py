@@ -144,7 +144,8 @@ class MoeLayer:
             self._raise(rc)
 
     def inject_device_status(self, status: int, stale_barrier_arrivals: int = 0):
-        """Host-side failure injection for tests of the error path (see the header)."""
+        """Host-side failure injection for tests of the error path (see the header); the second value goes into the
+        decode kernel's work counter (its name is from a form of the kernel that had grid barriers)."""
         stream = torch.cuda.current_stream(self.device).cuda_stream
         rc = self._lib.moe_fp8_b200_inject_device_status(self._h, int(status), int(stale_barrier_arrivals),
                                                          C.c_void_p(stream))
@@ -152,7 +153,8 @@ class MoeLayer:
             self._raise(rc)
 
     def invalidate_weights(self):
-        """Call after the weight-scale tensors' contents changed under the same addresses."""
+        """Call after the weight-scale tensors' contents changed under the same addresses (unless the scales are
+        read in place, see set_scales_in_place)."""
         rc = self._lib.moe_fp8_b200_invalidate_weights(self._h)
         if rc != _lib.OK:
             self._raise(rc)
@@ -325,8 +327,8 @@ class MoeLayer:
     def run_host(self, routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights,
                  gemm1_weights_scale, gemm2_weights, gemm2_weights_scale, local_expert_offset,
                  routed_scaling_factor, output, stream: Optional[int] = None):
-        """Per-call tensors (logits, hidden, hidden scale, output) in HOST memory; the call
-        copies in, runs, copies out and synchronises."""
+        """Per-call tensors (logits, hidden, hidden scale, output) in HOST memory; the call copies in, runs, copies
+        out and synchronises, or has the kernels read and write pinned buffers in place (see host_path)."""
         a = self._args(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights,
                        gemm1_weights_scale, gemm2_weights, gemm2_weights_scale, local_expert_offset,
                        routed_scaling_factor, output, host=True)

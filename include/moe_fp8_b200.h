@@ -136,9 +136,9 @@ enum {
     MOE_FP8_B200_BUF_SFA2 = 12,         /* fp32 [16, M_cap] */
     MOE_FP8_B200_BUF_Y = 13,            /* bf16 [M_cap, 7168] */
     MOE_FP8_B200_BUF_STATUS = 14,       /* int32 [2] device status word + detail */
-    MOE_FP8_B200_BUF_DECODE_TIMELINE = 15, /* uint64 [16] ns clock of CTA 0 in the last decode-kernel run: [0..6] start, tables
-                                           * built, phase 1 done, barrier 1 passed, phase 2 done, barrier 2 passed, end;
-                                           * [8..11] inside the table build: token routed, pairs listed, tables merged, published */
+    MOE_FP8_B200_BUF_DECODE_TIMELINE = 15, /* uint64 [16] ns clock of CTA 0 in the last decode-kernel run: [0..4] start, tables
+                                           * built, its phase 1 done, its first rows of phase 2 taken up, its last unit
+                                           * done; [5], [6] combine kernel's start and end; [8..11] inside the table build: token routed, pairs listed, tables merged, published */
     MOE_FP8_B200_BUF_EXCHANGE_TIMELINE = 16, /* uint64 [8] ns clock of the last moe_fp8_b200_run_reduce_scatter on this rank:
                                             * [0] push starts, [1] push done and flags published, [2] owner step starts
                                             * waiting for its peers, [3] all peers' flags seen, [4] owner step done */
@@ -164,7 +164,7 @@ MOE_FP8_B200_API int moe_fp8_b200_create(moe_fp8_b200_handle* out, int device, i
 
 /* Other shapes of the same layer.  The reference compiles hidden 7168 / intermediate 2048 and the routing
  * constants 8 / 8 / 4 in (kernel/moe_fp8.cu:292-304); FlashInfer's definition of the operator carries them
- * as axes.  A handle made here runs the five-kernel chain with those values at run time:
+ * as axes.  A handle made here runs the staged chain with those values at run time:
  *   hidden        multiple of 256, 256 .. 8192     tensors [T, hidden], scales [hidden/128, T]
  *   intermediate  multiple of 128, 128 .. 8192     W1 [E, 2*intermediate, hidden], W2 [E, hidden, intermediate]
  *   top_k         1 .. 8                            experts per token; table rows keep 8 entries, the unused ones
@@ -356,11 +356,11 @@ MOE_FP8_B200_API int moe_fp8_b200_check(moe_fp8_b200_handle h, void* stream);
 
 /* Failure injection FROM THE HOST, for tests of the error path (nothing on the GPU faults, traps or
  * hangs): writes `status` into the device status word as if a kernel had recorded it, and
- * `stale_barrier_arrivals` into the work counter of the decode kernel as a
+ * `stale_tickets` into the work counter of the decode kernel as a
  * launch that gave up half-way would leave it.  Synchronises `stream`.  No counterpart in the
  * reference, whose errors go to stderr only. */
 MOE_FP8_B200_API int moe_fp8_b200_inject_device_status(moe_fp8_b200_handle h, int status,
-                                                       unsigned stale_barrier_arrivals, void* stream);
+                                                       unsigned stale_tickets, void* stream);
 
 /* Mean device time in ms of the six stages (routing+dispatch, offset scan, permute, GEMM1,
  * GEMM2, combine) over the runs recorded since stage timing was switched on (at most the

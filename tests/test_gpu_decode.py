@@ -1,5 +1,5 @@
 """The single-kernel decode path (batches of at most 8 tokens, B200): against the CPU oracle,
-against the staged five-kernel chain on the same inputs, against the reference's GPU build, and
+against the staged chain on the same inputs, against the reference's GPU build, and
 its behaviour under CUDA graphs and repeated calls."""
 import numpy as np
 import pytest

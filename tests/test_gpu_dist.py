@@ -169,7 +169,7 @@ def _worker_varying_t(rank, world, port, q):
     dist.init_process_group("nccl", rank=rank, world_size=world, device_id=torch.device("cuda", rank))
     try:
         Tmax = 96
-        seq = [96, 33, 96, 40, 96, 12]   # all above 8 tokens: both forms then run the same five-kernel chain
+        seq = [96, 33, 96, 40, 96, 12]   # all above 8 tokens: both forms then run the same staged chain
         moe = ShardedMoe(Tmax)
         w = gen.make_shard(moe.local_expert_offset, moe.num_local_experts, device="cuda", out_device="cuda")
         cases, want = {}, {}

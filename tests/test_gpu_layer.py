@@ -664,7 +664,7 @@ def test_load_aware_expert_placement_sums_to_the_full_layer(pkg):
 # ------------------------------------------------------------------------- failure reporting
 def test_device_status_is_sticky_until_checked(pkg):
     """A failure that a kernel recorded survives later runs until the host reads it.  The failure is
-    injected from the host (a status word and a stale grid-barrier count copied into the control block, as
+    injected from the host (a status word and a stale work counter copied into the control block, as
     a decode launch that gave up half-way would leave them); nothing on the GPU faults or hangs.  Two more
     runs are enqueued, check() must still report the failure, and after it the next run is correct again."""
     T = 4
@@ -673,7 +673,7 @@ def test_device_status_is_sticky_until_checked(pkg):
     lay = pkg.MoeLayer(64, 32, 0)
     try:
         good = hp.run_layer(lay, inputs, weights, 0).clone()
-        for chain_T in (4, 40):    # the decode kernel (T <= 8) and the five-kernel chain
+        for chain_T in (4, 40):    # the decode kernel (T <= 8) and the staged chain
             inp = inputs if chain_T == 4 else hp.cpu_inputs(chain_T, seed=5001)
             want = hp.run_layer(lay, inp, weights, 0).clone()
             lay.inject_device_status(105, stale_barrier_arrivals=7)
