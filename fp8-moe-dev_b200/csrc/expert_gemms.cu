@@ -33,6 +33,7 @@
 //               into fp32 registers (arbitrary fp32 scales rule the block-scaled MMA kinds out); a thread
 //               owns one row and 128 of the 256 columns.  At the end of a unit's K loop they hand a bf16 tile
 //               over in shared memory and go on with the next unit
+// Host-resident calls whose output is written in place give a few CTAs another role (see zero_empty_rows).
 // Every wait is bounded; one that runs out sets the CTA's abort flag, all roles unwind, TMEM is released and
 // the failure is reported through Control::status.
 #include "gemm_tile.cuh"
@@ -123,6 +124,22 @@ __device__ __forceinline__ bool next_unit(FusedShared* sh, uint32_t ui, volatile
     return d.mode != 0;
 }
 
+// Output rows of the tokens that have no expert here (most of them where a GPU holds one shard of eight), written to
+// pinned host memory while the other CTAs' GEMMs run.  Behind the permute: beside it, its read requests would queue
+// behind these writes on their way out (host call on 32 experts, beside / behind: T=512 369 / 337 us, T=1024 520 /
+// 474).  Bound by PCIe, which few CTAs of plain stores fill (52 GB/s; cudaMemcpyAsync 56.7) if they do not share an SM:
+// as CTAs of this launch each has its own.  A warp per row.
+__device__ __forceinline__ void zero_empty_rows(const Workspace& ws, const EmptyRows& rows) {
+    const int lane = threadIdx.x & 31, warps = rows.ctas * (kGemmThreads / 32);
+    const bool none = ws.num_tiles[0] == 0;
+    const int vecs = ws.geo.hidden * 2 / 16;
+    for (int t = (int)blockIdx.x * (kGemmThreads / 32) + (int)(threadIdx.x >> 5); t < rows.T; t += warps) {
+        if (!none && ws.pair_count[t] != 0) continue;
+        uint4* row = reinterpret_cast<uint4*>(rows.out) + (size_t)t * vecs;
+        for (int i = lane; i < vecs; i += 32) row[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
 }  // namespace
 
 // GENERIC takes hidden / intermediate from Workspace::geo (hidden a multiple of 256, intermediate of 128, at
@@ -134,7 +151,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
     const __grid_constant__ CUtensorMap tmap_a1, const __grid_constant__ CUtensorMap tmap_w1,
     const __grid_constant__ CUtensorMap tmap_a2, const __grid_constant__ CUtensorMap tmap_w2,
     const __grid_constant__ CUtensorMap tmap_y, Workspace ws, const float* __restrict__ w1_scale,
-    const float* __restrict__ w2_scale, int silu_exact, int phases)
+    const float* __restrict__ w2_scale, int silu_exact, int phases, EmptyRows empty_rows)
 {
     static_assert(!(SMALLA && GENERIC), "the 64-row activation box is a variant of the reference's geometry");
     const int hidden = GENERIC ? ws.geo.hidden : kHidden;
@@ -155,6 +172,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) expert_gemms_kernel(
     const int lane = threadIdx.x & 31;
 
     pdl_launch_dependents();
+    if ((int)blockIdx.x < empty_rows.ctas) {   // whole CTAs, before any barrier or TMEM is set up
+        pdl_wait();
+        zero_empty_rows(ws, empty_rows);
+        return;
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&sh->full[s]), 1);
@@ -575,7 +597,8 @@ cudaError_t configure_expert_gemms()
 
 // `small_a` (reference geometry, at most 64 tokens): maps.a1 / maps.a2 are the 64-row views of the packed rows.
 cudaError_t launch_expert_gemms(const GemmMaps& maps, const Workspace& ws, const float* w1_scale, const float* w2_scale,
-                                int silu_exact, int phases, int num_ctas, int small_a, cudaStream_t stream)
+                                int silu_exact, int phases, int num_ctas, int small_a, const EmptyRows& empty_rows,
+                                cudaStream_t stream)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_ctas < 1 ? 1 : num_ctas);
@@ -590,7 +613,7 @@ cudaError_t launch_expert_gemms(const GemmMaps& maps, const Workspace& ws, const
     auto map = [](const void* p) { return *static_cast<const CUtensorMap*>(p); };
     auto go = [&](auto* kernel) {
         return cudaLaunchKernelEx(&cfg, kernel, map(maps.a1), map(maps.w1), map(maps.a2), map(maps.w2), map(maps.y), ws,
-                                  w1_scale, w2_scale, silu_exact, phases);
+                                  w1_scale, w2_scale, silu_exact, phases, empty_rows);
     };
     if (!ws.geo.is_reference()) return go(expert_gemms_kernel<true, false>);
     return small_a ? go(expert_gemms_kernel<false, true>) : go(expert_gemms_kernel<false, false>);

@@ -27,8 +27,6 @@ constexpr int kMaxLocalExperts = 256;
 // (one per work unit).
 constexpr int kSplitKSlots = 320;
 
-constexpr int kZeroCtas = 3;         // CTAs of zero_rows_kernel, and SMs that the GEMMs leave free beside it
-
 // What the dispatch step does with a token's experts that fall into one 32-expert
 // shard.  The fields restate, as data, the branch structure of the reference's
 // routing kernel (kernel/moe_fp8.cu:457-607) after its compile-time knobs
@@ -165,6 +163,13 @@ struct FetchList {
         seg[n].dst = static_cast<uint32_t*>(dst);
         seg[n++].words = bytes / 4;
     }
+};
+
+// Output rows of the tokens without an expert here that the expert GEMMs' launch writes beside its GEMMs (in the
+// first `ctas` of its CTAs; 0 = none).
+struct EmptyRows {
+    uint8_t* out;   // [T, hidden] bf16
+    int T, ctas;
 };
 
 // Tensor maps of one pair of GEMM launches (host addresses of CUtensorMap objects): packed activations and

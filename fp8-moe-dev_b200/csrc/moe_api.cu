@@ -19,7 +19,6 @@ cudaError_t launch_route_dispatch(const float*, const void*, const Workspace&, i
                                   const DispatchPolicy&, int, cudaStream_t);
 cudaError_t launch_permute(const void*, const float*, const Workspace&, int, cudaStream_t);
 cudaError_t launch_combine(const Workspace&, void*, int, int, int, cudaStream_t);
-cudaError_t launch_zero_rows(const Workspace&, void*, int, cudaStream_t);
 cudaError_t launch_fetch_inputs(const FetchList&, int, cudaStream_t);
 cudaError_t launch_quantize_rows(const void*, void*, float*, int, int, cudaStream_t);
 cudaError_t launch_combine_push(const Workspace&, const ExchangeView&, int, cudaStream_t);
@@ -33,7 +32,8 @@ size_t tensor_map_bytes();
 cudaError_t configure_gemm_kernels();
 cudaError_t launch_splitk_gemm(int, const GemmMaps&, const Workspace&, const float*, int, int, cudaStream_t);
 cudaError_t configure_expert_gemms();
-cudaError_t launch_expert_gemms(const GemmMaps&, const Workspace&, const float*, const float*, int, int, int, int, cudaStream_t);
+cudaError_t launch_expert_gemms(const GemmMaps&, const Workspace&, const float*, const float*, int, int, int, int, const EmptyRows&,
+                                cudaStream_t);
 size_t packed_scale_floats(int mode, int num_experts, const Geometry& geo);
 cudaError_t launch_repack_weight_scales(const float*, const float*, float*, float*, int, const Geometry&, cudaStream_t);
 cudaError_t launch_tile_weights(int, const void*, void*, int, const Geometry&, int, cudaStream_t);
@@ -51,6 +51,7 @@ constexpr int kVersion = (0 << 16) | 1;
 // experts T=128 355 / 353, T=256 426 / 440, T=2048 1192 / 1308; 128 experts T=1024 1243 / 1237).
 constexpr int kZeroAsideExperts = 64;
 constexpr int kZeroAsideTokens = 256;
+constexpr int kZeroCtas = 4;   // CTAs of the GEMMs' launch that write them
 // Half of the experts: nearly every row moves (few zero rows to leave early) and the permute and combine under which
 // transfers can hide are half as long as with all of them, so that a copy engine's 8 % higher rate wins, by little,
 // from about a thousand tokens on (us, copies / in place: T=256 752 / 741, T=512 938 / 924, T=1024 1240 / 1238, T=2048
@@ -182,9 +183,6 @@ struct moe_fp8_b200_ctx {
     uint8_t* stage = nullptr;
     size_t stage_bytes = 0;
     int host_path = 0;        // what the latest run_host did (moe_fp8_b200_host_path)
-    // run_host with pinned buffers: the rows without a local expert are written on a stream of their own
-    cudaStream_t side = nullptr;
-    cudaEvent_t side_begin = nullptr, side_done = nullptr;
     // pipelined host path: two staging sets, copy streams, per-set events
     uint8_t* pipe_stage[2] = {nullptr, nullptr};
     size_t pipe_bytes = 0;
@@ -234,8 +232,8 @@ void resolve_reference_policy(int T, DispatchPolicy& p)
     p.renorm = (T == 14107) ? 0 : 1;
 }
 
-// `zero_aside` (staged chain only, handle's side stream present): the output rows of tokens without a local expert
-// are written on the side stream while the GEMMs run, the combine leaves them out, and `stream` waits for both.
+// `zero_aside` (staged chain only): the output rows of tokens without a local expert are written by a few CTAs of the
+// GEMMs' launch, and the combine leaves them out.
 int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_t stream,
                   const ExchangeView* ex = nullptr, bool finalize = true, bool zero_aside = false)
 {
@@ -355,20 +353,14 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
     // at most 64 tokens (an expert then has at most 64 rows): 64-row activation boxes and a fourth operand stage
     const int small_a = (h->opt_small_batch_ring && T > 4 && T <= 64 && ref_geo) ? 1 : 0;
     if (e == cudaSuccess && stop >= 2) e = launch_permute(a.hidden_states, a.hidden_states_scale, h->ws, T, stream);
-    if (zero_aside) {
-        if (e == cudaSuccess) e = cudaEventRecord(h->side_begin, stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->side_begin, 0);
-        if (e == cudaSuccess) e = launch_zero_rows(h->ws, a.output, T, h->side);
-        if (e == cudaSuccess) e = cudaEventRecord(h->side_done, h->side);
-    }
     mark(3);
     const GemmMaps maps = {small_a ? h->tmap_a1_small : h->tmap_a1, tiled ? h->tmap_w1_tiled : h->tmap_w1,
                            small_a ? h->tmap_a2_small : h->tmap_a2, tiled ? h->tmap_w2_tiled : h->tmap_w2, h->tmap_y};
-    // one persistent CTA per SM (a CTA takes all of an SM's registers: some SMs are left to zero_rows_kernel where that
-    // runs); CTAs without work leave at once
-    const int gemm_ctas = zero_aside && h->num_sms > kZeroCtas ? h->num_sms - kZeroCtas : h->num_sms;
+    // one persistent CTA per SM; CTAs without work leave at once
     auto gemms = [&](int phases) {
-        return launch_expert_gemms(maps, gemm_ws, scale1, scale2, h->opt_exact_silu, phases, gemm_ctas, small_a, stream);
+        const EmptyRows empty = {static_cast<uint8_t*>(a.output), T, zero_aside && (phases & 1) ? kZeroCtas : 0};
+        return launch_expert_gemms(maps, gemm_ws, scale1, scale2, h->opt_exact_silu, phases,
+                                   h->num_sms > empty.ctas ? h->num_sms : empty.ctas + 1, small_a, empty, stream);
     };
     if (split_k) {
         if (e == cudaSuccess && stop >= 3)
@@ -392,7 +384,6 @@ int enqueue_layer(moe_fp8_b200_handle h, const moe_fp8_b200_args& a, cudaStream_
             e = launch_combine(h->ws, a.output, T, zero_aside ? 1 : 0, /*from_views=*/0, stream);
         }
     }
-    if (e == cudaSuccess && zero_aside) e = cudaStreamWaitEvent(stream, h->side_done, 0);
     mark(6);
     if (e != cudaSuccess) {
         h->counters_dirty = true;
@@ -642,9 +633,6 @@ int moe_fp8_b200_destroy(moe_fp8_b200_handle h)
         if (h->pipe_compute_done[i]) cudaEventDestroy(h->pipe_compute_done[i]);
         if (h->pipe_out_done[i]) cudaEventDestroy(h->pipe_out_done[i]);
     }
-    if (h->side_begin) cudaEventDestroy(h->side_begin);
-    if (h->side_done) cudaEventDestroy(h->side_done);
-    if (h->side) cudaStreamDestroy(h->side);
     if (h->pipe_in) cudaStreamDestroy(h->pipe_in);
     if (h->pipe_out) cudaStreamDestroy(h->pipe_out);
     if (h->w1_tiled) cudaFree(h->w1_tiled);
@@ -928,15 +916,6 @@ int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, 
     h->host_path = direct ? 2 : 1;
     if (direct) {
         const bool zero_aside = h->num_local_experts <= kZeroAsideExperts && T >= kZeroAsideTokens;
-        if (zero_aside && !h->side_done) {
-            int low = 0, high = 0;
-            e = cudaDeviceGetStreamPriorityRange(&low, &high);
-            // ahead of the combine's CTAs, which want the free SM as well
-            if (e == cudaSuccess && !h->side) e = cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, high);
-            if (e == cudaSuccess && !h->side_begin) e = cudaEventCreateWithFlags(&h->side_begin, cudaEventDisableTiming);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->side_done, cudaEventDisableTiming);
-            if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "side stream set-up: %s", cudaGetErrorString(e));
-        }
         FetchList list = {};
         list.add(p_logits, d_logits, n_logits);
         list.add(p_scale, d_scale, n_scale);
@@ -947,7 +926,6 @@ int moe_fp8_b200_run_host(moe_fp8_b200_handle h, const moe_fp8_b200_args* args, 
         if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "fetch of the host inputs: %s", cudaGetErrorString(e));
         const int rc = enqueue_layer(h, dev, stream, nullptr, true, zero_aside);
         // a call that failed half-way leaves nothing behind that still writes to the caller's memory
-        if (rc != MOE_FP8_B200_OK && zero_aside) cudaStreamSynchronize(h->side);
         if (rc != MOE_FP8_B200_OK) { cudaStreamSynchronize(stream); return rc; }
         e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return fail(h, MOE_FP8_B200_ERR_CUDA, "host-resident call: %s", cudaGetErrorString(e));

@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(Workspace ws, 
                              pairs.row[1].x, pairs.row[1].y, pairs.row[1].z, pairs.row[1].w};
     const float wts[kTopK] = {pairs.weight[0].x, pairs.weight[0].y, pairs.weight[0].z, pairs.weight[0].w,
                               pairs.weight[1].x, pairs.weight[1].y, pairs.weight[1].z, pairs.weight[1].w};
-    if (skip_empty && rows[0] < 0) return;   // zero_rows_kernel has that row
+    if (skip_empty && rows[0] < 0) return;   // the expert GEMMs' launch has written that row
     float acc[2][8];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(256) combine_generic_kernel(Workspace ws, __nv
                              pairs.row[1].x, pairs.row[1].y, pairs.row[1].z, pairs.row[1].w};
     const float wts[kTopK] = {pairs.weight[0].x, pairs.weight[0].y, pairs.weight[0].z, pairs.weight[0].w,
                               pairs.weight[1].x, pairs.weight[1].y, pairs.weight[1].z, pairs.weight[1].w};
-    if (skip_empty && rows[0] < 0) return;   // zero_rows_kernel has that row
+    if (skip_empty && rows[0] < 0) return;   // the expert GEMMs' launch has written that row
     const int H = ws.geo.hidden;
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)t * H);
     for (int v = threadIdx.x; v < H / 8; v += blockDim.x) {
@@ -466,33 +466,12 @@ __global__ void __launch_bounds__(kFetchThreads) fetch_inputs_kernel(const __gri
     }
 }
 
-// Output rows of the tokens that have no expert here (most of them where a GPU holds one shard of eight), written to
-// the host while the experts' GEMMs run, for which these leave an SM free per CTA.  On a stream of its own behind the
-// permute: not earlier, because the permute's read requests would queue behind these writes on their way out (host
-// call on 32 experts, beside the permute / behind it: T=512 369 / 337 us, T=1024 520 / 474), and by then the GEMMs'
-// CTAs hold all other SMs (the combine's, which would take the free ones, start behind the GEMMs in these calls).
-// Bound by PCIe, which few CTAs of plain stores fill if they do not share an SM (32 experts, T=1024 / 2048 / 4096, us:
-// four CTAs on one SM 440 / 810 / 1575, two on two 429 / 765 / 1491, three on three 423 / 765 / 1489, four on four
-// 425 / 764 / 1490).  A warp per row.
-constexpr int kZeroThreads = 512;
-__global__ void __launch_bounds__(kZeroThreads) zero_rows_kernel(Workspace ws, uint8_t* __restrict__ out, int T)
-{
-    const int lane = threadIdx.x & 31, warps = kZeroCtas * (kZeroThreads / 32);
-    const bool none = ws.num_tiles[0] == 0;
-    const int vecs = ws.geo.hidden * 2 / 16;
-    for (int t = blockIdx.x * (kZeroThreads / 32) + (threadIdx.x >> 5); t < T; t += warps) {
-        if (!none && ws.pair_count[t] != 0) continue;
-        uint4* row = reinterpret_cast<uint4*>(out) + (size_t)t * vecs;
-        for (int i = lane; i < vecs; i += 32) row[i] = make_uint4(0u, 0u, 0u, 0u);
-    }
-}
-
 // ---------------------------------------------------------------------------------------
-// Launchers (called by the C-ABI layer).  All launches but two carry the programmatic stream
-// serialization attribute (see ptx.cuh): zero_rows_kernel, and the combine beside it.
+// Launchers (called by the C-ABI layer).  All launches carry the programmatic stream
+// serialization attribute (see ptx.cuh).
 // ---------------------------------------------------------------------------------------
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_one(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args... args)
 {
     cudaLaunchConfig_t cfg = {};
@@ -504,13 +483,8 @@ static cudaError_t launch_one(bool early, void (*kernel)(KArgs...), dim3 grid, d
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = early ? 1 : 0;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)
-{
-    return launch_one(true, kernel, grid, block, smem, stream, args...);
 }
 
 cudaError_t launch_route_dispatch(const float* logits, const void* bias, const Workspace& ws, int T,
@@ -541,16 +515,10 @@ cudaError_t launch_combine(const Workspace& ws, void* out, int T, int skip_empty
 {
     __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
     if (!ws.geo.is_reference())
-        return launch_one(!skip_empty, from_views ? combine_generic_kernel<true> : combine_generic_kernel<false>, dim3(T),
-                          dim3(256), 0, stream, ws, o, T, skip_empty);
-    return launch_one(!skip_empty, from_views ? combine_kernel<true> : combine_kernel<false>, dim3(T), dim3(kCombineThreads), 0,
-                      stream, ws, o, T, skip_empty);
-}
-
-cudaError_t launch_zero_rows(const Workspace& ws, void* out, int T, cudaStream_t stream)
-{
-    zero_rows_kernel<<<kZeroCtas, kZeroThreads, 0, stream>>>(ws, static_cast<uint8_t*>(out), T);
-    return cudaGetLastError();
+        return launch_pdl(from_views ? combine_generic_kernel<true> : combine_generic_kernel<false>, dim3(T), dim3(256), 0, stream,
+                          ws, o, T, skip_empty);
+    return launch_pdl(from_views ? combine_kernel<true> : combine_kernel<false>, dim3(T), dim3(kCombineThreads), 0, stream, ws, o,
+                      T, skip_empty);
 }
 
 cudaError_t launch_fetch_inputs(const FetchList& list, int num_sms, cudaStream_t stream)
